@@ -72,7 +72,8 @@ struct cpg_handle {
   bool multi_graph = false;
   std::vector<int32_t> graph_voff;  // first vertex of each graph
   std::vector<int32_t> graph_from;  // per graph: lowest changed level (INT32_MAX: clean)
-  DevMem d_vgraph, d_graph_from, d_upd, d_queue, d_dl, d_long;
+  std::vector<ChangedGraph> changed;  // the graphs a rebuild walks
+  DevMem d_vgraph, d_graph_from, d_changed, d_upd, d_located, d_queue, d_dl, d_long;
   // side-by-side graphs relabelled in level order by cpg_batch_commit: the
   // caller's id of each vertex (device) and the new position of each of the
   // caller's edges (host, for delay updates); empty otherwise
@@ -90,7 +91,6 @@ struct cpg_handle {
   int32_t dirty_level = -1;  // lowest level whose delays changed
   std::vector<int32_t> h_level_of, h_succ;
   bool h_sfxt_cached = false;
-  bool h_levels_cached = false;  // levels depend on the graph, not on delays
   DevMem d_order, d_lvlp, d_level_of, d_dist, d_succ, d_dev_cnt, d_dev,
       d_ht_root, d_ht_size, d_hnodes, d_pool_mark, d_deps, d_sctr, d_best;
   unsigned long long hnode_cap = 0;
@@ -411,7 +411,6 @@ Status upload_graph(cpg_handle* h, int32_t n, int32_t m, const int32_t* adjp,
   h->has_graph = true;
   h->sfxt_valid = false;
   h->h_sfxt_cached = false;
-  h->h_levels_cached = false;
   h->dirty_level = -1;
   h->result_valid = false;
   h->n_result = 0;
@@ -514,7 +513,7 @@ Status load_edgelist(cpg_handle* h, const EdgeList& el) {
                  : upload_graph(h, g.n, g.m, g.adjp.data(), g.adj.data(), g.w.data());
 }
 
-SfxtParams sfxt_params(cpg_handle* h, int32_t start_level) {
+SfxtParams sfxt_params(cpg_handle* h, int32_t start_level, bool known = false) {
   SfxtParams p{};
   p.n = h->g.n;
   p.adjp = P<int32_t>(h->d_adjp);
@@ -566,6 +565,13 @@ SfxtParams sfxt_params(cpg_handle* h, int32_t start_level) {
       p.graph_from = P<int32_t>(h->d_graph_from);
     }
   }
+  if (known) {
+    p.known = 1;
+    if (start_level > 0 && h->multi_graph && h->relabeled) {
+      p.changed = P<ChangedGraph>(h->d_changed);
+      p.n_changed = static_cast<int32_t>(h->changed.size());
+    }
+  }
   if (h->use_bvss) {
     p.bvss = 1;
     p.bv_ptr = P<int32_t>(h->d_bv_ptr);
@@ -584,22 +590,33 @@ SfxtParams sfxt_params(cpg_handle* h, int32_t start_level) {
 }
 
 // Device work of one suffix-tree build, asynchronous and capturable.
+// known: the levels are an earlier build's (a rebuild after delay updates).
 Status enqueue_sfxt(cpg_handle* h, int32_t start_level, int* launches,
-                    bool kernel_events = false) {
+                    bool kernel_events = false, bool known = false) {
   cudaStream_t s = h->stream;
-  if (h->multi_graph && start_level > 0)
+  if (h->multi_graph && start_level > 0) {
     CK(cudaMemcpyAsync(h->d_graph_from.p, h->graph_from.data(), h->graph_from.size() * 4,
                        cudaMemcpyHostToDevice, s), "H2D changed levels");
+    if (known && h->relabeled) {
+      h->changed.clear();
+      for (size_t g = 0; g < h->graph_from.size(); ++g)
+        if (h->graph_from[g] != INT32_MAX)
+          h->changed.push_back({h->graph_voff[g], h->graph_voff[g + 1], h->graph_from[g], 0});
+      CK(cudaMemcpyAsync(h->d_changed.p, h->changed.data(),
+                         h->changed.size() * sizeof(ChangedGraph), cudaMemcpyHostToDevice, s),
+         "H2D changed graphs");
+    }
+  }
   CK(launch_init_sfxt_counters(P<SfxtCounters>(h->d_sctr), P<unsigned long long>(h->d_pool_mark),
                                start_level, start_level > 0, s),
      "sfxt counters");
-  if (h->use_bvss && start_level == 0) {
+  if (h->use_bvss && start_level == 0 && !known) {
     // the pull leaves the bitmaps clear; a build cut short by an error may not
     CK(cudaMemsetAsync(h->d_fbits.p, 0, h->d_fbits.bytes, s), "memset");
     CK(cudaMemsetAsync(h->d_iact.p, 0, h->d_iact.bytes, s), "memset");
   }
   int grid = 0;
-  CK(launch_sfxt(sfxt_params(h, start_level), h->device, s, &grid, launches,
+  CK(launch_sfxt(sfxt_params(h, start_level, known), h->device, s, &grid, launches,
                  kernel_events ? h->ev[6] : nullptr, kernel_events ? h->ev[7] : nullptr),
      "sfxt launch");
   *launches += 1;
@@ -607,7 +624,7 @@ Status enqueue_sfxt(cpg_handle* h, int32_t start_level, int* launches,
 }
 
 // Reads the build's counters back; kRetry when the heap pool overflowed.
-int finish_sfxt(cpg_handle* h, int32_t start_level) {
+int finish_sfxt(cpg_handle* h, int32_t start_level, bool known = false) {
   SfxtCounters* out = static_cast<SfxtCounters*>(h->pinned);
   CK(cudaMemcpyAsync(out, h->d_sctr.p, sizeof(SfxtCounters), cudaMemcpyDeviceToHost, h->stream),
      "D2H sfxt counters");
@@ -615,16 +632,13 @@ int finish_sfxt(cpg_handle* h, int32_t start_level) {
   if (out->err == kDevTimeout)
     return fail(h, CPG_ERR_TIMEOUT, "suffix tree: grid barrier wait ran out");
   if (out->err == kDevCapacity) return kRetry;
-  if (start_level == 0) {
+  if (start_level == 0 && !known) {
     h->levels = out->levels;
-    h->h_levels_cached = false;
-  }
-  h->stats.levels = h->levels;
-  if (start_level == 0) {
     h->stats.frontier_used = h->use_bvss ? CPG_FRONTIER_BVSS : CPG_FRONTIER_CSR;
     h->stats.bvss_tiles_tensor = static_cast<int64_t>(out->vss_tensor);
     h->stats.bvss_tiles_scalar = static_cast<int64_t>(out->vss_scalar);
   }
+  h->stats.levels = h->levels;
   h->stats.bvss_bits_per_slice = h->bvss_bps;
   h->sfxt_valid = true;
   h->h_sfxt_cached = false;
@@ -640,16 +654,16 @@ Status grow_heap_pool(cpg_handle* h) {
   return CPG_OK;
 }
 
-Status run_sfxt(cpg_handle* h, int32_t start_level) {
+Status run_sfxt(cpg_handle* h, int32_t start_level, bool known = false) {
   cudaStream_t s = h->stream;
   for (int attempt = 0; attempt < 8; ++attempt) {
     CK(cudaEventRecord(h->ev[0], s), "event");
     int launches = 0;
-    Status st = enqueue_sfxt(h, start_level, &launches, true);
+    Status st = enqueue_sfxt(h, start_level, &launches, true, known);
     if (st != CPG_OK) return st;
     CK(cudaEventRecord(h->ev[1], s), "event");
     h->stats.kernel_launches += launches;
-    const int r = finish_sfxt(h, start_level);
+    const int r = finish_sfxt(h, start_level, known);
     float ms = 0.f, kms = 0.f;
     cudaEventElapsedTime(&ms, h->ev[0], h->ev[1]);
     cudaEventElapsedTime(&kms, h->ev[6], h->ev[7]);
@@ -685,26 +699,21 @@ Status cache_sfxt_host(cpg_handle* h) {
   return CPG_OK;
 }
 
-// Host copy of the reverse levels (kept across delay updates).
-Status ensure_levels_host(cpg_handle* h) {
-  if (h->h_levels_cached) return CPG_OK;
-  const size_t n = h->g.n;
-  h->h_level_of.resize(n);
-  if (n)
-    CK(cudaMemcpy(h->h_level_of.data(), h->d_level_of.p, n * 4, cudaMemcpyDeviceToHost), "D2H levels");
-  h->h_levels_cached = true;
-  return CPG_OK;
-}
-
 Status ensure_sfxt(cpg_handle* h) {
   {
     Status st = ready_graph(h);
     if (st != CPG_OK) return st;
   }
   if (h->sfxt_valid) return CPG_OK;
-  if (h->dirty_level > 0 && h->levels > 0)
-    return run_sfxt(h, h->dirty_level);
-  return run_sfxt(h, 0);
+  if (h->dirty_level <= 0 || h->levels <= 0) return run_sfxt(h, 0);
+  if (h->opts.sfxt_level_sync == 1) return run_sfxt(h, h->dirty_level);
+  // The levels are known.  A rebuild from a level on appends its chain heaps
+  // to the pool, which has room for about half a tree more; one that reaches
+  // down to the lowest quarter of the levels rebuilds the few others too and
+  // starts the pool afresh, instead of overflowing it every second time and
+  // rebuilding everything then.
+  const bool all = !h->multi_graph && h->dirty_level < h->levels / 4;
+  return run_sfxt(h, all ? 0 : h->dirty_level, true);
 }
 
 struct Counts {
@@ -1300,7 +1309,7 @@ cpg_status cpg_destroy(cpg_handle* h) {
                    &h->d_qids, &h->d_ehist, &h->d_esort, &h->d_equery, &h->d_ectr,
                    &h->d_bv_ptr, &h->d_bv_masks, &h->d_bv_rows, &h->d_bv_cnt,
                    &h->d_bv_deps, &h->d_fbits, &h->d_iact, &h->d_act_list,
-                   &h->d_vgraph, &h->d_graph_from, &h->d_upd, &h->d_queue, &h->d_dl,
+                   &h->d_vgraph, &h->d_graph_from, &h->d_changed, &h->d_upd, &h->d_located, &h->d_queue, &h->d_dl,
                    &h->d_long, &h->d_orig_id};
   for (DevMem* b : all) release(*b);
   for (auto& e : h->ev)
@@ -1437,40 +1446,37 @@ cpg_status cpg_update_delays(cpg_handle* h, int64_t count, const int32_t* eids,
     }
     eids = mapped.data();
   }
-  int32_t lowest = INT32_MAX;
+  // The device checks the ids and finds the changed tails' lowest level per
+  // graph, then writes the delays.  Staging kept by the handle: no allocation
+  // (and no device-wide synchronisation) per update.
   const bool have_levels = h->sfxt_valid || h->dirty_level > 0;
-  if (have_levels) {
-    Status st = ensure_levels_host(h);
-    if (st != CPG_OK) return st;
-  }
-  // tail of each fan-out edge, by binary search over the CSR offsets
-  for (int64_t i = 0; i < count; ++i) {
-    const int32_t e = eids[i];
-    if (e < 0 || e >= h->g.m) return fail(h, CPG_ERR_INVALID, "edge id out of range");
-  }
-  for (int64_t i = 0; have_levels && i < count; ++i) {
-    const auto it = std::upper_bound(h->g.adjp.begin(), h->g.adjp.end(), eids[i]);
-    const int32_t tail = static_cast<int32_t>(it - h->g.adjp.begin()) - 1;
-    const int32_t lv = h->h_level_of[tail];
-    if (lv < 0) continue;
-    lowest = std::min(lowest, lv);
-    if (h->multi_graph) {
-      const size_t g = static_cast<size_t>(
-          std::upper_bound(h->graph_voff.begin(), h->graph_voff.end(), tail) -
-          h->graph_voff.begin() - 1);
-      h->graph_from[g] = std::min(h->graph_from[g], lv);
-    }
-  }
-  // staging kept by the handle: no allocation (and no device-wide
-  // synchronisation) per update
+  const size_t ng = h->multi_graph ? h->graph_from.size() : 1;
   CK(ensure_grow(h->d_upd, static_cast<size_t>(count) * 8), "alloc delay update");
+  CK(ensure_grow(h->d_located, (ng + 1) * 4), "alloc delay update");
   int32_t* up_e = P<int32_t>(h->d_upd);
   float* up_w = reinterpret_cast<float*>(up_e + count);
   CK(cudaMemcpyAsync(up_e, eids, count * 4, cudaMemcpyHostToDevice, h->stream), "H2D eids");
   CK(cudaMemcpyAsync(up_w, w, count * 4, cudaMemcpyHostToDevice, h->stream), "H2D delays");
-  CK(launch_scatter_delays(P<DevEdge>(h->d_edges), up_e, up_w, count, h->stream),
-     "scatter delays");
-  CK(cudaStreamSynchronize(h->stream), "scatter delays");
+  SfxtParams up = sfxt_params(h, 0);
+  up.vgraph = h->multi_graph ? P<int32_t>(h->d_vgraph) : nullptr;
+  CK(launch_update_delays(up, P<DevEdge>(h->d_edges), h->g.m, up_e, up_w, count, have_levels,
+                          P<int32_t>(h->d_located), static_cast<int32_t>(ng), h->stream),
+     "delay update");
+  std::vector<int32_t> far;  // more graphs than the pinned staging holds
+  int32_t* located = static_cast<int32_t*>(h->pinned);
+  if ((ng + 1) * 4 > kPinnedBytes) {
+    far.resize(ng + 1);
+    located = far.data();
+  }
+  CK(cudaMemcpyAsync(located, h->d_located.p, (ng + 1) * 4, cudaMemcpyDeviceToHost, h->stream),
+     "D2H changed levels");
+  CK(cudaStreamSynchronize(h->stream), "delay update");
+  if (located[0] != 0) return fail(h, CPG_ERR_INVALID, "edge id out of range");
+  int32_t lowest = INT32_MAX;
+  for (size_t g = 0; g < ng; ++g) {
+    lowest = std::min(lowest, located[1 + g]);
+    if (h->multi_graph) h->graph_from[g] = std::min(h->graph_from[g], located[1 + g]);
+  }
   // incremental rebuild from the lowest changed level (levels never change
   // with delays); without levels a full rebuild follows
   if (have_levels && lowest != INT32_MAX && lowest >= 1)
@@ -2039,6 +2045,8 @@ cpg_status cpg_batch_commit(cpg_batch* b) {
       std::fill(vg.begin() + b->voff[g], vg.begin() + b->voff[g + 1], static_cast<int32_t>(g));
     CK(ensure(h->d_vgraph, std::max<size_t>(vg.size(), 1) * 4), "alloc graph ids");
     CK(ensure(h->d_graph_from, std::max<size_t>(ng, 1) * 4), "alloc graph ids");
+    CK(ensure(h->d_changed, std::max<size_t>(ng, 1) * sizeof(ChangedGraph)), "alloc graph ids");
+    CK(ensure(h->d_located, (ng + 1) * 4), "alloc graph ids");
     if (n)
       CK(cudaMemcpy(h->d_vgraph.p, vg.data(), vg.size() * 4, cudaMemcpyHostToDevice), "H2D graph ids");
   }

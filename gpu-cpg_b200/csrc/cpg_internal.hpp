@@ -137,6 +137,12 @@ struct SfxtCounters {
 // read back whole into the handle's 4 KiB pinned staging
 static_assert(sizeof(SfxtCounters) <= 4096, "SfxtCounters outgrew the pinned staging");
 
+// One side-by-side graph with changed delays: its id range and the lowest
+// level a change touches.
+struct ChangedGraph {
+  int32_t v_beg, v_end, from, pad;
+};
+
 struct SfxtParams {
   int32_t n;
   const int32_t* adjp;
@@ -174,6 +180,13 @@ struct SfxtParams {
   const int32_t* vgraph;
   const int32_t* graph_from;
   int32_t append_pool;
+  // Rebuild over levels an earlier build found (sfxt_known_kernel): no Kahn
+  // step.  The vertices come from order[] (levels start_level on), or, with
+  // changed set, from n_changed side-by-side graphs relabelled in level
+  // order, each graph's own id range from its lowest changed level on.
+  int32_t known;
+  const ChangedGraph* changed;
+  int32_t n_changed;
   // full CSR builds: dataflow work queue (n ints) unless level_sync is set
   int32_t* queue;
   int32_t* long_rows;      // rows over 64 edges, written unsorted (n ints)
@@ -495,8 +508,9 @@ int launch_topk_costs(const float* costs, unsigned long long n, unsigned long lo
                       const TopkScratch& s, float* out, unsigned long long* n_out,
                       void* stream);
 
-// Scatter new delays into the device fan-out edges.
-int launch_scatter_delays(DevEdge* edges, const int32_t* eids, const float* w,
-                          int64_t count, void* stream);
+// Checks, locates (lowest changed level per graph) and writes new delays.
+int launch_update_delays(const SfxtParams& p, DevEdge* edges, int32_t m, const int32_t* eids,
+                         const float* w, int64_t count, bool have_levels, int32_t* out,
+                         int32_t ng, void* stream);
 
 }  // namespace cpg
