@@ -1133,6 +1133,20 @@ __device__ __forceinline__ unsigned long long ld_dl(const SfxtParams& p, int h) 
   return *reinterpret_cast<const volatile unsigned long long*>(p.dl + h);
 }
 
+// Publishes v's (level, dist) word.  It carries everything a tail's build
+// reads of v, so it needs no fence before it and goes out as soon as the
+// distance is known, before v's successor and deviation row: the chain of
+// words from level to level bounds the walk over known levels (kernel 0.131 ->
+// 0.096 ms on 20,000 pins, 0.374 -> 0.348 ms on 200,000, 1.53 -> 1.37 ms on 1M;
+// the dataflow build of the 1M-pin graph 1.69 -> 1.66 ms, at degree 50 2.16 ->
+// 2.11 ms, of smaller graphs the same).  All lanes call.
+__device__ __forceinline__ void publish_dl(const SfxtParams& p, int v, int lvl, int best) {
+  if ((threadIdx.x & 31) == 0)
+    *reinterpret_cast<volatile unsigned long long*>(p.dl + v) =
+        (static_cast<unsigned long long>(static_cast<unsigned>(lvl)) << 32) |
+        static_cast<unsigned>(best);
+}
+
 __device__ int build_vertex_polled(const SfxtParams& p, int v, int rb, int re, DevEdge ed0,
                                    unsigned long long dl0) {
   const int lane = threadIdx.x & 31;
@@ -1196,11 +1210,13 @@ __device__ int build_vertex_polled(const SfxtParams& p, int v, int rb, int re, D
     const int lvl = warp_max_i(lmax) + 1;
     if (lvl == 0) {
       best = 0;  // a sink
+      publish_dl(p, v, lvl, best);
     } else {
 #pragma unroll
       for (int c = 0; c < kRegChunks; ++c)
         if (ed[c].head >= 0) best = min(best, cand_dist(dh[c], ed[c].w));
       best = warp_min_i(best);
+      publish_dl(p, v, lvl, best);
       int nt = 0;  // this lane's tied heads
 #pragma unroll
       for (int c = 0; c < kRegChunks; ++c)
@@ -1312,6 +1328,7 @@ __device__ int build_vertex_polled(const SfxtParams& p, int v, int rb, int re, D
     if (!__all_sync(0xffffffffu, ok)) return -1;
     const int lvl = warp_max_i(lmax) + 1;
     best = warp_min_i(lbest);
+    publish_dl(p, v, lvl, best);
     s = warp_max_i(lbest == best ? ls : -1);
     // the heads' distances come from their published words
     auto dist_of = [&](int h) { return static_cast<int>(ld_dl(p, h) & 0xffffffffu); };
@@ -1364,11 +1381,6 @@ __device__ int build_vertex_polled(const SfxtParams& p, int v, int rb, int re, D
     if (re - rb > 64 && cnt > 1 && cnt <= kSmemRow) list_long_row(p, v);
     if (cnt > 0) p.best[v] = top;
     p.level_of[v] = lmax;
-    // the word carries everything a tail's build reads of v, so it needs
-    // no fence before it
-    *reinterpret_cast<volatile unsigned long long*>(p.dl + v) =
-        (static_cast<unsigned long long>(static_cast<unsigned>(lmax)) << 32) |
-        static_cast<unsigned>(best);
   }
   return lmax;
 }
@@ -1765,10 +1777,10 @@ sfxt_dataflow_kernel(SfxtParams p) {
 //
 // What bounds it is the chain of published words from level to level and,
 // on large graphs, the warps' round trips per vertex.  With every level
-// rebuilt it takes 0.37 ms on 200,000 pins and 122 levels (3 us a level),
+// rebuilt it takes 0.35 ms on 200,000 pins and 122 levels (2.9 us a level),
 // against 2.82 ms with one grid barrier per level (23 us a level: a build's
 // and a heap insert's chain of loads each) and 0.57 ms for the dataflow
-// build, which finds the levels again; 1.54 against 1.70 ms on 1M pins.
+// build, which finds the levels again; 1.37 against 1.66 ms on 1M pins.
 // Heaps in a phase of their own below the line: 0.71 ms on 200,000 pins.
 //
 // Side-by-side graphs (p.changed) are walked at the same time, graph
