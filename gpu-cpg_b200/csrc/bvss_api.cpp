@@ -398,14 +398,6 @@ cpg_status cpg_bvss_discover_pairs(cpg_bvss* b, const cpg_bvss_opts* opts,
     stats->mma_issued = static_cast<int64_t>(c.mma_issued);
     stats->device_ms = ms;
   }
-  // (u, v) order, as the reference returns them
-  std::vector<std::pair<int32_t, int32_t>> pv(static_cast<size_t>(got));
-  for (int64_t i = 0; i < got; ++i) pv[i] = {pairs[2 * i], pairs[2 * i + 1]};
-  std::sort(pv.begin(), pv.end());
-  for (int64_t i = 0; i < got; ++i) {
-    pairs[2 * i] = pv[i].first;
-    pairs[2 * i + 1] = pv[i].second;
-  }
   if (total > max_pairs) return bfail(b, CPG_ERR_CAPACITY, "BVSS pairs: more pairs than max_pairs");
   return CPG_OK;
 }

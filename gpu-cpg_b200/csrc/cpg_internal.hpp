@@ -281,10 +281,15 @@ int launch_bvss_levels(const DevBvss& b, const int32_t* sinks, int32_t n_sinks,
                        int32_t* levels, unsigned int* scratch, BvssCounters* ctr,
                        BvssDispatch d, unsigned int spin_limit, int device, void* stream);
 // Pairs (source u in the frontier, row v) of an A_dev BVSS.
+// Sorted by (u, v); the first max_pairs of them are written.
 size_t bvss_pairs_scratch_words(int32_t n_intervals, int32_t n_vss);
 int launch_bvss_pairs(const DevBvss& b, const int32_t* sources, int32_t n_sources,
                       int32_t* pairs, long long max_pairs, unsigned int* scratch,
                       BvssCounters* ctr, BvssDispatch d, void* stream);
+
+// Exclusive prefix sums (graph_build.cu); sums: scan_scratch_words(n) ints.
+size_t scan_scratch_words(int64_t n);
+void launch_exclusive_scan(const int32_t* x, int64_t n, int32_t* y, int32_t* sums, void* stream);
 
 constexpr int kSfxtThreads = 1024;  // one block per SM: fewer grid-barrier arrivals
 constexpr int kSmemRow = 256;  // deviation rows up to this length sort in smem

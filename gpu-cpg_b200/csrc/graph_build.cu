@@ -32,8 +32,8 @@ __global__ void interleave_indegree_kernel(const int32_t* adj, const float* w, i
   }
 }
 
-// exclusive scan of x[0..n) into y[0..n], y[n] = total; three-kernel
-// reduce-then-scan over kScanTile-element tiles
+// exclusive scan of x[0..n) into y[0..n], y[n] = total (launch_exclusive_scan);
+// three-kernel reduce-then-scan over kScanTile-element tiles
 __global__ void tile_sum_kernel(const int32_t* x, int64_t n, int32_t* sums) {
   __shared__ int32_t ws[32];
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile;
@@ -90,7 +90,6 @@ __global__ void __launch_bounds__(1024) scan_sums_kernel(int32_t* sums, int n) {
 
 __global__ void tile_scan_kernel(const int32_t* x, int64_t n, const int32_t* sums,
                                  int32_t* y) {
-  __shared__ int32_t buf[kScanTile];
   __shared__ int32_t wsum[32];
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile;
   constexpr int per = kScanTile / 256;  // blockDim.x == 256
@@ -125,11 +124,7 @@ __global__ void tile_scan_kernel(const int32_t* x, int64_t n, const int32_t* sum
     if (g < n) y[g] = pre;
     pre += vals[i];
   }
-  (void)buf;
-}
-
-__global__ void set_last_kernel(int32_t* y, int64_t n, const int32_t* sums, int ntiles) {
-  y[n] = sums[ntiles];
+  if (blockIdx.x == 0 && threadIdx.x == 0) y[n] = sums[gridDim.x];
 }
 
 // warp per tail vertex: each fan-out edge (u, h) lands in h's fan-in row
@@ -169,6 +164,20 @@ int grid_of(int64_t n, int threads) {
 
 }  // namespace
 
+size_t scan_scratch_words(int64_t n) {
+  return static_cast<size_t>((n + kScanTile - 1) / kScanTile + 1);
+}
+
+// y[0..n) = exclusive prefix sums of x[0..n), y[n] = their total (n > 0; y
+// may be x).  sums: scan_scratch_words(n) ints.
+void launch_exclusive_scan(const int32_t* x, int64_t n, int32_t* y, int32_t* sums, void* stream) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int ntiles = static_cast<int>((n + kScanTile - 1) / kScanTile);
+  tile_sum_kernel<<<ntiles, 256, 0, s>>>(x, n, sums);
+  scan_sums_kernel<<<1, 1024, 0, s>>>(sums, ntiles);
+  tile_scan_kernel<<<ntiles, 256, 0, s>>>(x, n, sums, y);
+}
+
 size_t build_scratch_words(int32_t n) {
   // indeg/fill (n) + tile sums
   return static_cast<size_t>(n) + (static_cast<size_t>(n) + kScanTile) / kScanTile + 2;
@@ -184,17 +193,13 @@ int launch_build_graph(const int32_t* adjp, const int32_t* adj, const float* w,
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int32_t* indeg = scratch;
   int32_t* sums = scratch + n;
-  const int ntiles = static_cast<int>((static_cast<int64_t>(n) + kScanTile - 1) / kScanTile);
   cudaMemsetAsync(indeg, 0, static_cast<size_t>(n) * 4, s);
   cudaMemsetAsync(n_srcs, 0, 8, s);  // source count, bad-head flag
   if (m > 0)
     interleave_indegree_kernel<<<grid_of(m, 256), 256, 0, s>>>(adj, w, m, n, edges, indeg,
                                                                n_srcs + 1);
   if (n > 0) {
-    tile_sum_kernel<<<ntiles, 256, 0, s>>>(indeg, n, sums);
-    scan_sums_kernel<<<1, 1024, 0, s>>>(sums, ntiles);
-    tile_scan_kernel<<<ntiles, 256, 0, s>>>(indeg, n, sums, iadjp);
-    set_last_kernel<<<1, 1, 0, s>>>(iadjp, n, sums, ntiles);
+    launch_exclusive_scan(indeg, n, iadjp, sums, stream);
     sources_kernel<<<grid_of(n, 256), 256, 0, s>>>(indeg, n, srcs, n_srcs);
     // reuse indeg as the scatter cursor
     cudaMemcpyAsync(indeg, iadjp, static_cast<size_t>(n) * 4, cudaMemcpyDeviceToDevice, s);

@@ -157,3 +157,33 @@ def test_sfxt_bvss_repeat_and_incremental():
         g.report_paths(500)
         h.report_paths(500)
         assert np.array_equal(g.get_slacks(500).view(np.uint32), h.get_slacks(500).view(np.uint32))
+
+
+@pytest.mark.parametrize("tiles", TILES)
+@pytest.mark.parametrize("n,hub,n_src", [(1, 1, 1), (9, 3, 9), (130, 129, 130), (1000, 700, 37),
+                                         (4099, 4000, 4099)])
+def test_pairs_come_in_order_over_intervals_of_several_vss(n, hub, n_src, tiles):
+    """Intervals with none, one and many VSS (a hub with `hub` heads), empty
+    rows and rows without a successor; the pairs that fit are the first."""
+    rng = np.random.default_rng(n + hub)
+    rows = [np.sort(rng.choice(n, size=min(n, int(rng.integers(0, 6))), replace=False))
+            for _ in range(n)]
+    rows[n // 2] = np.sort(rng.choice(n, size=hub, replace=False))
+    adjp = np.concatenate([[0], np.cumsum([r.size for r in rows])]).astype(np.int32)
+    adj = np.concatenate(rows).astype(np.int32)
+    succ = np.array([r[-1] if r.size and u % 3 else -1 for u, r in enumerate(rows)], np.int32)
+    sources = rng.permutation(n)[:n_src].astype(np.int32)
+    want = oracle.adev_pairs(n, adjp, adj, succ, sources)
+    b = cpg_b200.Bvss(n, adjp, adj, succ)
+    got, _ = b.discover_pairs(sources, max_pairs=want.shape[0] + 3, tiles=tiles)
+    np.testing.assert_array_equal(got, want)
+    buf, total = np.full(2 * max(want.shape[0], 1), -7, np.int32), cpg_b200.C.c_int64()
+    few = want.shape[0] // 2
+    o = cpg_b200.Bvss._opts(0, tiles, 0, 0, 0, None)
+    st = cpg_b200.lib.cpg_bvss_discover_pairs(
+        b._b, cpg_b200.C.byref(o), cpg_b200._ptr(sources), sources.size, cpg_b200._ptr(buf), few,
+        cpg_b200.C.byref(total), None)
+    assert total.value == want.shape[0]
+    assert st == (4 if few < want.shape[0] else 0)
+    np.testing.assert_array_equal(buf[:2 * few].reshape(-1, 2), want[:few])
+    assert (buf[2 * few:] == -7).all()
