@@ -37,8 +37,15 @@ struct DevMem {
 constexpr unsigned int kDefaultSpinLimit = 1u << 24;
 // the handle's pinned staging of counters and small tables
 constexpr size_t kPinnedBytes = 4096;
-// single queries: pending items up to which one CTA runs a phase
+// pending items up to which a query's block runs its phases
 constexpr unsigned long long kEngSoloStop = 4096;
+// k up to which a block answers a query to the end.  Alone on the device it
+// is ahead of the grid launch up to about 4,000 (1M-pin graph: 0.147 against
+// 0.212 ms at k = 1,000, 0.322 against 0.347 at 4,000; one CTA of the grid
+// launch takes 0.64 against 0.36 ms at 8,000).  Beside other queries, which
+// keep the other SMs busy, up to what its sort buffer holds: 48 served
+// requests of k up to 20,000 take 6.3 ms, against 9.8 ms in grid launches.
+constexpr long long kWholeAlone = 4096, kWholeBeside = kBlockMaxK;
 enum { kRetry = 1000 };  // internal: a bounded buffer overflowed, grow and rerun
 constexpr int32_t kMaxRow = 16384;  // longest deviation row the row sort takes
 
@@ -114,6 +121,10 @@ struct cpg_handle {
   int sfxt_grid_limit = 0;
   int engine_grid_limit = 0;
   int sel_schedule = 0;  // 0: 11/11/10-bit select digits, 1: 8/8/8/8
+  // the prepared queries: whether any goes on to the grid launch, and the
+  // grid's part of the path store and the piles
+  bool engine_grid_part = false;
+  unsigned long long grid_paths = 0, grid_pend = 0, grid_front = 0;
 
   // staging
   void* pinned = nullptr;
@@ -1022,11 +1033,53 @@ int try_query(cpg_handle* h, unsigned long long k) {
 // (asynchronous and capturable: memsets and one cooperative launch) and
 // finish (read counters back, map errors).
 
+// Which queries their blocks answer whole, where each query's costs go, and
+// every block's share of the path store and piles: in proportion to k, the
+// queries that go on to the grid launch first, so that the grid's part of
+// each is one range from 0.
+void engine_layout(cpg_handle* h, std::vector<EngineQuery>& qs) {
+  const long long whole_max = h->opts.engine_ctas > 0 ? 0 : qs.size() > 1 ? kWholeBeside : kWholeAlone;
+  auto weight = [](const EngineQuery& q) {
+    return static_cast<unsigned long long>(std::max<long long>(q.k, 64)) +
+           static_cast<unsigned long long>(q.src_end - q.src_beg);
+  };
+  unsigned long long all = 0, off = 0, at = 0;
+  for (EngineQuery& q : qs) {
+    q.whole = q.k <= whole_max;
+    q.out_off = off;
+    off += static_cast<unsigned long long>(q.k);
+    all += weight(q);
+  }
+  auto part = [&](unsigned long long cap, unsigned long long w) {
+    return static_cast<unsigned long long>(static_cast<unsigned __int128>(cap) * w / all);
+  };
+  h->engine_grid_part = false;
+  for (const int whole : {0, 1}) {
+    for (EngineQuery& q : qs) {
+      if (q.whole != whole) continue;
+      const unsigned long long end = at + weight(q);
+      q.path_base = part(h->cap_paths, at);
+      q.path_cap = part(h->cap_paths, end) - q.path_base;
+      q.pend_base = part(h->cap_pend, at);
+      q.pend_cap = part(h->cap_pend, end) - q.pend_base;
+      q.front_base = part(h->cap_front, at);
+      q.front_cap = part(h->cap_front, end) - q.front_base;
+      at = end;
+      if (!whole) h->engine_grid_part = true;
+    }
+    if (!whole) {
+      h->grid_paths = part(h->cap_paths, at);
+      h->grid_pend = part(h->cap_pend, at);
+      h->grid_front = part(h->cap_front, at);
+    }
+  }
+}
+
 // Buffers for nq queries whose K sum to k_total.
-Status engine_prepare(cpg_handle* h, const std::vector<EngineQuery>& qs,
-                      unsigned long long k_total) {
+Status engine_prepare(cpg_handle* h, std::vector<EngineQuery> qs, unsigned long long k_total) {
   Status st = alloc_query(h, k_total);
   if (st != CPG_OK) return st;
+  engine_layout(h, qs);
   int grid = 0;
   CK(engine_grid(h->device, h->engine_grid_limit, &grid), "engine occupancy");
   const size_t nq = qs.size();
@@ -1049,20 +1102,21 @@ Status engine_prepare(cpg_handle* h, const std::vector<EngineQuery>& qs,
   return CPG_OK;
 }
 
-// solo_stop > 0 (single queries): a one-CTA launch runs the phases while the
-// pending pile holds at most solo_stop items, then the launch on the handle's
-// CTA count resumes where it stopped (or finds the query answered and
-// returns).  *launches receives the number of launches.
+// One launch with a block per query, then, unless the blocks answer every
+// query whole, the grid launch on the handle's CTA count, which goes on with
+// what they left.  *launches receives the number of launches.
 Status engine_enqueue(cpg_handle* h, int nq, unsigned long long k_total,
-                      unsigned long long solo_stop = 0, int* launches = nullptr) {
+                      int* launches = nullptr) {
   cudaStream_t s = h->stream;
   int grid = 0;
   CK(engine_grid(h->device, h->engine_grid_limit, &grid), "engine occupancy");
   CK(cudaMemsetAsync(h->d_ectr.p, 0, sizeof(EngineCounters), s), "memset");
-  CK(cudaMemsetAsync(h->d_ehist.p, 0, static_cast<size_t>(nq) * kSelBins * 4, s), "memset");
-  // every output slot is written by the compaction; zero-filling keeps a path
-  // index in range even if selection and compaction ever disagreed
-  CK(cudaMemsetAsync(h->d_vals.p, 0, 2 * k_total * 4, s), "memset");
+  if (h->engine_grid_part) {
+    CK(cudaMemsetAsync(h->d_ehist.p, 0, static_cast<size_t>(nq) * kSelBins * 4, s), "memset");
+    // every output slot is written by the compaction; zero-filling keeps a path
+    // index in range even if selection and compaction ever disagreed
+    CK(cudaMemsetAsync(h->d_vals.p, 0, 2 * k_total * 4, s), "memset");
+  }
   EngineParams p{};
   p.g.adjp = P<int32_t>(h->d_adjp);
   p.g.dist = P<int32_t>(h->d_dist);
@@ -1076,13 +1130,14 @@ Status engine_enqueue(cpg_handle* h, int nq, unsigned long long k_total,
   p.nq = nq;
   p.root_ref = h->opts.root_seeding == CPG_ROOTS_REFERENCE;
   p.ps = path_store(h);
+  p.ps.cap = h->grid_paths;
   p.pq = P<int32_t>(h->d_pq);
   p.pend[0] = P<Item>(h->d_pend0);
   p.pend[1] = P<Item>(h->d_pend1);
-  p.pend_cap = h->cap_pend;
+  p.pend_cap = h->grid_pend;
   p.front[0] = P<Item>(h->d_front0);
   p.front[1] = P<Item>(h->d_front1);
-  p.front_cap = h->cap_front;
+  p.front_cap = h->grid_front;
   p.hist = P<unsigned int>(h->d_ehist);
   p.keys[0] = P<unsigned int>(h->d_keys);
   p.keys[1] = P<unsigned int>(h->d_keys) + k_total;
@@ -1095,7 +1150,8 @@ Status engine_enqueue(cpg_handle* h, int nq, unsigned long long k_total,
   p.digit_tot = P<unsigned int>(h->d_esort) + 256 * static_cast<size_t>(grid);
   p.rank_of = P<int32_t>(h->d_rank);
   p.out_cost = P<float>(h->d_out_cost);
-  p.out_nodes = P<cpg_path_node>(h->d_out_nodes);
+  // side-by-side graphs (batched and served forms) return costs only
+  p.out_nodes = h->multi_graph ? nullptr : P<cpg_path_node>(h->d_out_nodes);
   p.ctr = P<EngineCounters>(h->d_ectr);
   p.spin_limit = h->opts.spin_limit ? h->opts.spin_limit : kDefaultSpinLimit;
   p.grid_limit = h->engine_grid_limit;
@@ -1112,18 +1168,10 @@ Status engine_enqueue(cpg_handle* h, int nq, unsigned long long k_total,
     p.sel_shift[1] = 10; p.sel_bits[1] = 11;
     p.sel_shift[2] = 0;  p.sel_bits[2] = 10;
   }
-  if (solo_stop > 0 && grid > 1) {
-    EngineParams a = p;
-    a.grid_limit = 1;
-    a.solo_stop = solo_stop;
-    CK(launch_engine(a, h->device, s), "engine launch");
-    p.resume = 1;
-    CK(launch_engine(p, h->device, s), "engine launch");
-    if (launches) *launches = 2;
-    return CPG_OK;
-  }
-  CK(launch_engine(p, h->device, s), "engine launch");
-  if (launches) *launches = 1;
+  p.solo_stop = kEngSoloStop;
+  CK(launch_engine_blocks(p, s), "engine launch");
+  if (h->engine_grid_part) CK(launch_engine(p, h->device, s), "engine launch");
+  if (launches) *launches = h->engine_grid_part ? 2 : 1;
   return CPG_OK;
 }
 
@@ -1155,6 +1203,8 @@ int engine_finish(cpg_handle* h, std::vector<EngineQuery>& qout, EngineCounters&
   else
     CK(cudaMemcpy(qout.data(), h->d_equery.p, nq * sizeof(EngineQuery), cudaMemcpyDeviceToHost),
        "D2H queries");
+  c.paths += c.blk_paths;
+  c.pend_out += c.blk_pend;
   h->stats.paths_accepted = static_cast<int64_t>(c.paths);
   h->stats.items_generated = static_cast<int64_t>(c.paths + c.pend_out);
   h->stats.pending_peak = static_cast<int64_t>(c.pend_out);
@@ -1169,18 +1219,14 @@ int engine_finish(cpg_handle* h, std::vector<EngineQuery>& qout, EngineCounters&
 // One query through the engine.  Returns kRetry when a bounded buffer
 // overflowed.
 int engine_query(cpg_handle* h, unsigned long long k) {
-  // CTAs of the engine launch: the option, else chosen from K (a small
-  // query's phases are bound by barrier latency, and one CTA's grid barrier
-  // is a block barrier)
-  // (measured on the 20,000-pin and 1M-pin graphs: one CTA is fastest up to
-  // K of about 2,000 -- 0.33 against 0.61 ms at K = 1,000 -- eight around
-  // K = 1e4, then about K / 3,000, up to one per SM at K = 1e6)
+  // CTAs of the grid launch, which goes on with what the query's block leaves:
+  // the option, else chosen from K, since more CTAs cost barrier latency and
+  // fewer cost throughput (1M-pin graph, 8 / 16 / 32 / 64 CTAs: 0.53 / 0.45 /
+  // 0.44 / 0.46 ms at k = 16,000, 0.74 / 0.62 / 0.57 / 0.57 ms at 40,000; about
+  // K / 3,000 above that, one per SM at 1e6)
   int ctas = h->opts.engine_ctas;
-  if (ctas <= 0) {
-    if (k <= 2000) ctas = 1;
-    else if (k <= 20000) ctas = 8;
-    else ctas = static_cast<int>(std::min<unsigned long long>(std::max<unsigned long long>(k / 3000, 16), 1u << 20));
-  }
+  if (ctas <= 0)
+    ctas = static_cast<int>(std::min<unsigned long long>(std::max<unsigned long long>(k / 3000, 32), 1u << 20));
   h->engine_grid_limit = ctas;  // engine_grid caps it at the co-resident CTAs
   std::vector<EngineQuery> qs(1);
   qs[0].k = static_cast<long long>(k);
@@ -1190,10 +1236,8 @@ int engine_query(cpg_handle* h, unsigned long long k) {
   if (st != CPG_OK) return st;
   cudaStream_t s = h->stream;
   CK(cudaEventRecord(h->ev[2], s), "event");
-  // the first phases move a few thousand items at most: one CTA runs them
-  // on block barriers, the full launch takes over once the pile is larger
   int launches = 0;
-  st = engine_enqueue(h, 1, k, kEngSoloStop, &launches);
+  st = engine_enqueue(h, 1, k, &launches);
   if (st != CPG_OK) return st;
   CK(cudaEventRecord(h->ev[3], s), "event");
   h->stats.kernel_launches += launches;

@@ -388,8 +388,12 @@ struct EngineQuery {
   unsigned long long pend_next_n, pend_next_nz;      // the pile being written
   unsigned long long k_out, out_off, out_lt, out_eq;
   int phases;
-  int pad;
+  int whole;                  // answered by its own block (engine_block_kernel)
   unsigned long long acc_prev, last_j;  // accepted before / promoted in the last growth phase
+  // set by the host: where the query's costs go, and its block's share of the
+  // path store and of the global overflow of its piles
+  unsigned long long path_base, path_cap, pend_base, pend_cap, front_base, front_cap;
+  unsigned long long seg_off;  // the grid's output: its segment of the sorted paths
 };
 
 struct EngineCounters {
@@ -410,9 +414,9 @@ struct EngineCounters {
   int rounds;
   int phases;
   int sorted_buf;             // which vals[] holds the sorted path indices
-  int stopped;                // a one-CTA launch stopped at phase res_phase
-  int res_phase, res_pin;     // the phase to resume and which pending pile is in
-  unsigned long long res_paths, res_pend;
+  int stopped;                // a block left its query to the grid launch
+  int res_phase;              // ... after this many phases at most
+  unsigned long long blk_paths, blk_pend;  // paths and pending items of the whole queries
   // device time per stage (ns): 0 seed, 1 decide/bookkeeping, 2 select,
   // 3 promote, 4 closure, 5 output select, 6 output sort, 7 emit
   unsigned long long t_ns[8];
@@ -445,11 +449,9 @@ struct EngineParams {
   unsigned int spin_limit;
   int grid_limit;             // persistent CTAs (0: one per co-resident slot)
   int grow_cap_k;             // cap a growth phase's promotion at K - accepted
-  // Two launches for a single query: a one-CTA launch runs the phases while
-  // the pending pile holds at most solo_stop items and stops there (state in
-  // EngineCounters::res_*); the full launch (resume = 1) continues.
+  // a block leaves a query that is not `whole` to the grid launch once more
+  // items than this are pending
   unsigned long long solo_stop;
-  int resume;
   int sel_passes;             // radix select digit schedule (sum of bits 32)
   int sel_shift[4];
   int sel_bits[4];
@@ -459,6 +461,11 @@ struct EngineParams {
 // host sizes sort_hist as 256 * grid) for a given CTA limit (0: maximum).
 int engine_grid(int device, int limit, int* grid_out);
 int launch_engine(const EngineParams& p, int device, void* stream);
+// One block per query: runs `whole` queries to the end and the others' first
+// phases (engine_block_kernel).
+int launch_engine_blocks(const EngineParams& p, void* stream);
+// Largest k a block answers whole: its sort buffer.
+constexpr long long kBlockMaxK = 16384;
 constexpr int kInlineQueries = 8;
 int launch_set_queries(EngineQuery* dst, const EngineQuery* src, int nq, void* stream);
 

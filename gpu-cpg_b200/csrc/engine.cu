@@ -203,12 +203,13 @@ __device__ __forceinline__ void qadd(EngineQuery* qs, size_t off, bool on, unsig
 #define QOFF(field) offsetof(EngineQuery, field)
 
 // ------------------------------------------------------------------ seeding
-// One warp per query: reachable sources become root items; with the
-// reference rule, roots at or below the initial split beyond the first
-// (int)(0.005f*R + 1) (in source-id order) are dropped.
-__device__ void seed_query(const EngineParams& p, int qi) {
+// One warp: reachable sources become root items, handed to put(keep, item)
+// 32 at a time (all lanes call it); with the reference rule, roots at or
+// below the initial split beyond the first (int)(0.005f*R + 1) (in source-id
+// order) are dropped.
+template <typename F>
+__device__ void seed_query(const EngineParams& p, int qi, EngineQuery& Q, F&& put) {
   const int lane = threadIdx.x & 31;
-  EngineQuery& Q = p.q[qi];
   const int b = Q.src_beg, e = Q.src_end;
   // number of reachable sources
   int r = 0;
@@ -263,19 +264,12 @@ __device__ void seed_query(const EngineParams& p, int qi) {
     kept_n += __popc(__ballot_sync(0xffffffffu, keep));
     kept_nz += __popc(__ballot_sync(0xffffffffu, keep && c != 0.0f));
     if (keep) rabs = fmaxf(rabs, fabsf(c));
-    const unsigned long long slot = warp_append(&p.ctr->pend_out, keep);
-    if (keep) {
-      if (slot < p.pend_cap) {
-        Item it;
-        it.cost = c;
-        it.parent = -1;
-        it.node = -2 - src;
-        it.j = pack_j(static_cast<unsigned>(qi), 0);
-        p.pend[0][slot] = it;
-      } else {
-        eng_fail(p, kDevCapacity);
-      }
-    }
+    Item it;
+    it.cost = c;
+    it.parent = -1;
+    it.node = -2 - src;
+    it.j = pack_j(static_cast<unsigned>(qi), 0);
+    put(keep, it);
   }
   for (int o = 16; o > 0; o >>= 1) rabs = fmaxf(rabs, __shfl_xor_sync(0xffffffffu, rabs, o));
   if (lane == 0) {
@@ -354,9 +348,10 @@ __device__ void select_hist(const EngineParams& p, unsigned long long n_paths,
   }
 }
 
-// select_pick for a single query by a whole block: each thread sums its
-// share of the bins, a block scan finds the share holding the krem-th key,
+// select_pick for a single query by a whole block (histogram in global or,
+// kShared, in shared memory): each thread sums its share of the bins, a block scan finds the share holding the krem-th key,
 // and its thread walks its few bins.  Each thread then clears its own bins.
+template <bool kShared>
 __device__ __noinline__ void select_pick_block(EngineQuery* q0, unsigned int* h, int shift,
                                                int bits, unsigned int* chosen_n) {
   __shared__ unsigned long long s_wsum[kEngWarps];
@@ -371,7 +366,7 @@ __device__ __noinline__ void select_pick_block(EngineQuery* q0, unsigned int* h,
 #pragma unroll
   for (int t = 0; t < 2; ++t)
     if (t < per && b0 + t < bins) {
-      mine[t] = __ldcg(h + b0 + t);
+      mine[t] = kShared ? h[b0 + t] : __ldcg(h + b0 + t);
       sum += mine[t];
     }
   // inclusive scan over the block, in thread (= bin) order
@@ -457,25 +452,36 @@ __device__ void select_pick(const EngineParams& p, int shift, int bits, int gw, 
   }
 }
 
-// D. The split and acceptance limit of every selecting query (threads t0,
-// t0 + nt, ...), and the cursors the promotion starts from.
+// A growth phase needs only about j items promoted, not the j-th exactly:
+// when the bin holding it is small against j, the split is the bin's upper
+// edge and the last pass is skipped.
+__device__ __forceinline__ bool coarse_split(const EngineQuery& Q, unsigned int bin_n) {
+  return Q.mode == 1 &&
+         static_cast<unsigned long long>(bin_n) <= (Q.ksel / 8 > 256 ? Q.ksel / 8 : 256ull);
+}
+
+// The split and acceptance limit of one selecting query.
+__device__ __forceinline__ void set_limit(EngineQuery& Q) {
+  const float t = key_float(Q.prefix);
+  Q.t = t;
+  if (Q.mode == 2) {
+    const float a = fmaxf(fmaxf(fabsf(t), Q.root_abs), 1.0f);
+    Q.lim = t + a * 0x1p-16f;
+    Q.tie = t;
+  } else {
+    // accept strictly below the split when anything pending is cheaper
+    // than it (ksel - krem items are), so a tie group at the split waits;
+    // a coarse split is a bin's upper edge and takes the whole bin
+    Q.lim = (Q.ksel > Q.krem && !Q.coarse) ? float_below(t) : t;
+    Q.tie = __int_as_float(0x7fc00000);  // NaN: expand every path
+  }
+}
+
+// D. The limits of every selecting query (threads t0, t0 + nt, ...), and the
+// cursors the promotion starts from.
 __device__ void set_limits(const EngineParams& p, unsigned t0, unsigned nt, bool reset) {
   for (unsigned qi = t0; qi < static_cast<unsigned>(p.nq); qi += nt) {
-    EngineQuery& Q = p.q[qi];
-    if (Q.mode == 0) continue;
-    const float t = key_float(Q.prefix);
-    Q.t = t;
-    if (Q.mode == 2) {
-      const float a = fmaxf(fmaxf(fabsf(t), Q.root_abs), 1.0f);
-      Q.lim = t + a * 0x1p-16f;
-      Q.tie = t;
-    } else {
-      // accept strictly below the split when anything pending is cheaper
-      // than it (ksel - krem items are), so a tie group at the split waits;
-      // a coarse split is a bin's upper edge and takes the whole bin
-      Q.lim = (Q.ksel > Q.krem && !Q.coarse) ? float_below(t) : t;
-      Q.tie = __int_as_float(0x7fc00000);  // NaN: expand every path
-    }
+    if (p.q[qi].mode != 0) set_limit(p.q[qi]);
   }
   if (reset) {
     p.ctr->frontier[0] = 0;
@@ -501,15 +507,10 @@ __device__ bool run_select(const EngineParams& p, unsigned long long n_paths,
       if (!eng_sync_last(p, [&]() {
             bool done = last;
             if (p.nq == 1) {
-              select_pick_block(p.q, p.hist, shift, bits, &s_chosen_n);
+              select_pick_block<false>(p.q, p.hist, shift, bits, &s_chosen_n);
               __syncthreads();
-              // A growth phase needs only about j items promoted, not the
-              // j-th exactly: when the bin holding it is small against j,
-              // split at the bin's upper edge and skip the last pass.
               EngineQuery& Q = p.q[0];
-              if (with_limits && pass == p.sel_passes - 2 && Q.mode == 1 &&
-                  static_cast<unsigned long long>(s_chosen_n) <=
-                      (Q.ksel / 8 > 256 ? Q.ksel / 8 : 256ull)) {
+              if (with_limits && pass == p.sel_passes - 2 && coarse_split(Q, s_chosen_n)) {
                 __syncthreads();  // every thread has read the query's mode
                 if (threadIdx.x == 0) {
                   Q.prefix |= (1u << shift) - 1u;
@@ -597,6 +598,99 @@ __device__ __forceinline__ unsigned long long warp_reserve(unsigned long long* c
   return base + (incl - n);
 }
 
+// An accepted item as a path, and its (up to) five children: heap left /
+// right (or row 2j+1 / 2j+2), row entries 1 and 2 of a heap node's row, and
+// the cross child.
+struct Grown {
+  HeapNode hn;
+  int cross;
+  float cc[5];
+  unsigned tm, dm;  // children at or below the limit, and above it
+  bool stored;
+};
+
+// Stores the path in slot qp (below cap) and prices the children.  Every
+// load is issued before the path's stores: what bounds a round is the chain
+// item -> node -> (row entry ->) heap of the path's head -> its root node.
+__device__ __forceinline__ Grown grow_path(const EngineParams& p, const Item& it, bool valid,
+                                           unsigned q, unsigned long long qp,
+                                           unsigned long long cap, float lim, float tie) {
+  Grown g;
+  const int jj = j_of(it);
+  g.hn.vtx = -1;
+  g.hn.left = -1;
+  g.hn.right = -1;
+  g.hn.row = 0;
+  g.hn.head = -1;
+  g.hn.w = 0.f;
+  g.hn.dist_head = 0;
+  g.hn.dist_v = 0;
+  g.stored = valid && qp < cap;
+  if (valid && !g.stored) eng_fail(p, kDevCapacity);
+  const bool dev = g.stored && it.node >= 0;
+  int to = -1, from = -1, level = 0;
+  float pcost = 0.f;
+  if (dev) {
+    g.hn = load_node(p.g.hnodes, it.node);
+    level = __ldcg(p.ps.level + it.parent) + 1;
+    pcost = __ldcg(p.ps.cost + it.parent);
+    from = g.hn.vtx;
+    to = dev_head(p.g, g.hn, jj);
+  } else if (g.stored) {
+    to = -(it.node + 2);
+  }
+  // a path costing exactly the final split is reported, not expanded
+  const bool expand = g.stored && !(it.cost == tie);
+  const bool sib = expand && dev;
+  g.cross = expand ? __ldg(p.g.ht_root + to) : -1;
+  // (the item's own node carries its row start, and every node the
+  // record of its element, so no child costs more than one more load)
+  unsigned exm = 0;
+  if (sib && (jj == 0 ? cand_top(p.g, g.hn.left, pcost, g.cc[0])
+                      : cand_row(p.g, g.hn, 2 * jj + 1, pcost, g.cc[0]))) exm |= 1u;
+  if (sib && (jj == 0 ? cand_top(p.g, g.hn.right, pcost, g.cc[1])
+                      : cand_row(p.g, g.hn, 2 * jj + 2, pcost, g.cc[1]))) exm |= 2u;
+  if (sib && jj == 0 && cand_row(p.g, g.hn, 1, pcost, g.cc[2])) exm |= 4u;
+  if (sib && jj == 0 && cand_row(p.g, g.hn, 2, pcost, g.cc[3])) exm |= 8u;
+  if (expand && cand_top(p.g, g.cross, it.cost, g.cc[4])) exm |= 16u;
+  g.tm = g.dm = 0;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    if (!(exm & (1u << k))) continue;
+    if (g.cc[k] <= lim) g.tm |= 1u << k;
+    else g.dm |= 1u << k;
+  }
+  if (g.stored) {
+    p.ps.cost[qp] = it.cost;
+    p.ps.parent[qp] = it.parent;
+    p.ps.from[qp] = from;
+    p.ps.to[qp] = to;
+    p.ps.level[qp] = level;
+    p.pq[qp] = static_cast<int>(q);
+  }
+  return g;
+}
+
+// Child k of an item grown into path qp.
+__device__ __forceinline__ Item child_of(const Grown& g, const Item& it, unsigned q,
+                                         unsigned long long qp, int k) {
+  const int jj = j_of(it);
+  Item c;
+  c.cost = g.cc[k];
+  c.parent = k == 4 ? static_cast<int>(qp) : it.parent;
+  c.node = k == 4 ? g.cross : (k < 2 && jj == 0 ? (k == 0 ? g.hn.left : g.hn.right) : it.node);
+  c.j = pack_j(q, k == 4 ? 0 : k == 2 ? 1 : k == 3 ? 2 : (jj == 0 ? 0 : 2 * jj + 1 + k));
+  return c;
+}
+
+// The pending children whose cost is not zero.
+__device__ __forceinline__ unsigned pending_nz(const Grown& g) {
+  unsigned n = 0;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) n += ((g.dm >> k) & 1u) && g.cc[k] != 0.0f;
+  return n;
+}
+
 // Rounds over the frontier until it is empty.  Returns false on error.
 __device__ bool run_closure(const EngineParams& p, Item* pend_out) {
   const unsigned long long tid =
@@ -629,89 +723,21 @@ __device__ bool run_closure(const EngineParams& p, Item* pend_out) {
       it.j = 0;
       if (valid) it = load_item(in, i);
       const unsigned q = q_of(it);
-      const int jj = j_of(it);
       const unsigned long long qp = warp_append(&p.ctr->paths, valid);
-      bool stored = false;
-      int to = -1;
-      HeapNode hn;
-      hn.vtx = -1;
-      hn.left = -1;
-      hn.right = -1;
-      hn.row = 0;
-      hn.head = -1;
-      hn.w = 0.f;
-      hn.dist_head = 0;
-      hn.dist_v = 0;
-      float lim = 0.f, tie = 0.f;
-      if (valid) {
-        lim = single ? lim0 : __ldcg(&p.q[q].lim);
-        tie = single ? tie0 : __ldcg(&p.q[q].tie);
-        int from = -1, level = 0;
-        if (it.node <= -2) {
-          to = -(it.node + 2);
-        } else {
-          hn = load_node(p.g.hnodes, it.node);
-          from = hn.vtx;
-          to = dev_head(p.g, hn, jj);
-          level = __ldcg(p.ps.level + it.parent) + 1;
-        }
-        if (qp < p.ps.cap) {
-          p.ps.cost[qp] = it.cost;
-          p.ps.parent[qp] = it.parent;
-          p.ps.from[qp] = from;
-          p.ps.to[qp] = to;
-          p.ps.level[qp] = level;
-          p.pq[qp] = static_cast<int>(q);
-          stored = true;
-        } else {
-          eng_fail(p, kDevCapacity);
-        }
-      }
-      if (single) acc_nz += stored && it.cost != 0.0f;
-      else qadd(p.q, QOFF(paths_nz), stored && it.cost != 0.0f, q, 1u);
-      // a path costing exactly the final split is reported, not expanded
-      const bool expand = stored && !(it.cost == tie);
-      const bool sib = expand && it.node >= 0;
-      const float pcost = sib ? __ldcg(p.ps.cost + it.parent) : 0.f;
-      // the (up to) five children: heap left / right (or row 2j+1 / 2j+2),
-      // row entries 1 and 2 of a heap node's row, and the cross child
-      const int cross = expand ? __ldg(p.g.ht_root + to) : -1;
-      float cc[5];
-      unsigned exm = 0;
-      // (the item's own node carries its row start, and every node the
-      // record of its element, so no child costs more than one more load)
-      if (sib && (jj == 0 ? cand_top(p.g, hn.left, pcost, cc[0])
-                          : cand_row(p.g, hn, 2 * jj + 1, pcost, cc[0]))) exm |= 1u;
-      if (sib && (jj == 0 ? cand_top(p.g, hn.right, pcost, cc[1])
-                          : cand_row(p.g, hn, 2 * jj + 2, pcost, cc[1]))) exm |= 2u;
-      if (sib && jj == 0 && cand_row(p.g, hn, 1, pcost, cc[2])) exm |= 4u;
-      if (sib && jj == 0 && cand_row(p.g, hn, 2, pcost, cc[3])) exm |= 8u;
-      if (expand && cand_top(p.g, cross, it.cost, cc[4])) exm |= 16u;
-      unsigned tm = 0, dm = 0, dnz = 0;
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        if (!(exm & (1u << k))) continue;
-        if (cc[k] <= lim) tm |= 1u << k;
-        else {
-          dm |= 1u << k;
-          dnz += cc[k] != 0.0f;
-        }
-      }
+      const Grown g = grow_path(p, it, valid, q, qp, p.ps.cap,
+                                single || !valid ? lim0 : __ldcg(&p.q[q].lim),
+                                single || !valid ? tie0 : __ldcg(&p.q[q].tie));
+      if (single) acc_nz += g.stored && it.cost != 0.0f;
+      else qadd(p.q, QOFF(paths_nz), g.stored && it.cost != 0.0f, q, 1u);
       // one reservation per warp and counter for all five
-      unsigned long long bt = warp_reserve(out_cnt, __popc(tm));
-      unsigned long long bd = warp_reserve(&p.ctr->pend_out, __popc(dm));
+      unsigned long long bt = warp_reserve(out_cnt, __popc(g.tm));
+      unsigned long long bd = warp_reserve(&p.ctr->pend_out, __popc(g.dm));
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
         const unsigned bit = 1u << k;
-        if (!((tm | dm) & bit)) continue;
-        Item c;
-        c.cost = cc[k];
-        c.parent = k == 4 ? static_cast<int>(qp) : it.parent;
-        const int cn = k == 4 ? cross : (k < 2 && jj == 0 ? (k == 0 ? hn.left : hn.right) : it.node);
-        const int cj = k == 4 ? 0 : k == 2 ? 1 : k == 3 ? 2 : (jj == 0 ? 0 : 2 * jj + 1 + k);
-        c.node = cn;
-        c.j = pack_j(q, cj);
-        if (tm & bit) {
+        if (!((g.tm | g.dm) & bit)) continue;
+        const Item c = child_of(g, it, q, qp, k);
+        if (g.tm & bit) {
           if (bt < p.front_cap) out[bt] = c;
           else eng_fail(p, kDevCapacity);
           ++bt;
@@ -721,7 +747,7 @@ __device__ bool run_closure(const EngineParams& p, Item* pend_out) {
           ++bd;
         }
       }
-      const unsigned ndef = __popc(dm), ndef_nz = dnz;
+      const unsigned ndef = __popc(g.dm), ndef_nz = pending_nz(g);
       if (single) {
         acc_pn += ndef;
         acc_pnz += ndef_nz;
@@ -858,7 +884,6 @@ __device__ bool decide_query(const EngineParams& p, EngineQuery& Q) {
     Q.mode = 2;                       // final: the k-th of paths+pending
     Q.krem = static_cast<unsigned long long>(Q.k);
     Q.ksel = Q.krem;
-    atomicOr(&p.ctr->sel_paths, 1);
   } else if (Q.pend_n > 0) {
     Q.mode = 1;                       // grow by count
     // promote ~4x the accepted count, but never more than half the
@@ -925,6 +950,7 @@ __device__ void next_phase(const EngineParams& p, int phase, bool finish) {
       Q.pend_next_n = Q.pend_next_nz = 0;
     }
     if (decide_query(p, Q)) atomicAdd(&p.ctr->active, 1);
+    if (Q.mode == 2) atomicOr(&p.ctr->sel_paths, 1);
   }
 }
 
@@ -933,50 +959,26 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
   const unsigned long long tid =
       static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   const unsigned long long nth = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
-  const int gw = static_cast<int>(tid >> 5);
-  const int nw = static_cast<int>(nth >> 5);
-
   unsigned long long t_last = 0;
   if (threadIdx.x == 0) s_stage = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) t_last = gtime();
-  int pin = 0, phase0 = 0;
-  unsigned long long n_pend = 0, n_paths = 0;
-  if (p.resume) {
-    // the one-CTA launch before this one either finished the query or
-    // stopped at the top of a phase; an error there ends this launch too
-    if (*reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk ||
-        !*reinterpret_cast<volatile int*>(&p.ctr->stopped))
-      return;
-    pin = __ldcg(&p.ctr->res_pin);
-    phase0 = __ldcg(&p.ctr->res_phase);
-    n_pend = __ldcg(&p.ctr->res_pend);
-    n_paths = __ldcg(&p.ctr->res_paths);
-  } else {
-    // seed roots (pending pile 0)
-    for (int qi = gw; qi < p.nq; qi += nw) seed_query(p, qi);
-    if (!eng_sync_last(p, [&]() { next_phase(p, 0, false); }))
-      return;
-    STAMP(0);
-    n_pend = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->pend_out);
-  }
+  // the blocks (engine_block_kernel) ran every query's first phases; what
+  // they left to the grid is in pile 0.  An error there ends this launch too.
+  if (*reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk ||
+      !*reinterpret_cast<volatile int*>(&p.ctr->stopped))
+    return;
+  if (!eng_sync_last(p, [&]() { next_phase(p, 0, false); })) return;
+  int pin = 0;
+  const int phase0 = __ldcg(&p.ctr->res_phase);
+  unsigned long long n_pend = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->pend_out);
+  unsigned long long n_paths = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->paths);
+  STAMP(0);
 
   for (int phase = phase0;; ++phase) {
     const Item* pend = p.pend[pin];
     Item* pend_next = p.pend[pin ^ 1];
     // (per-query counts are kept current by seeding, promotion and closure)
     if (*reinterpret_cast<volatile int*>(&p.ctr->active) == 0) break;
-    if (p.solo_stop && n_pend > p.solo_stop) {
-      // the pile outgrew one CTA: leave the rest to the full launch
-      if (threadIdx.x == 0) {
-        p.ctr->res_pin = pin;
-        p.ctr->res_phase = phase;
-        p.ctr->res_pend = n_pend;
-        p.ctr->res_paths = n_paths;
-        p.ctr->stopped = 1;
-        __threadfence();
-      }
-      return;
-    }
     // C + D. per-query radix select, split and acceptance limit
     if (!run_select(p, n_paths, pend, n_pend, true)) return;
     STAMP(2);
@@ -1111,7 +1113,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         EngineQuery& W = p.q[0];
         W.k_out = k_out;
-        W.out_off = 0;
+        W.seg_off = 0;
         W.mode = k_out > 0 ? 3 : 0;
         p.ctr->out_total = k_out;
       }
@@ -1125,6 +1127,10 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
     ENG_SYNC();
     for (unsigned long long qi = tid; qi < static_cast<unsigned long long>(p.nq); qi += nth) {
       EngineQuery& Q = p.q[qi];
+      if (Q.whole) {  // its block wrote its output
+        Q.mode = 0;
+        continue;
+      }
       const unsigned long long k = static_cast<unsigned long long>(Q.k);
       Q.k_out = Q.paths_nz < k ? Q.paths_nz : k;
       Q.mode = Q.k_out > 0 ? 3 : 0;
@@ -1137,7 +1143,8 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       unsigned long long acc = 0;
       for (int qi = 0; qi < p.nq; ++qi) {
-        p.q[qi].out_off = acc;
+        if (p.q[qi].whole) continue;
+        p.q[qi].seg_off = acc;
         acc += p.q[qi].k_out;
       }
       p.ctr->out_total = acc;
@@ -1180,7 +1187,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
           const EngineQuery& Q = p.q[q];
           const unsigned long long need_eq = __ldcg(&Q.krem);
           const unsigned long long n_lt = __ldcg(&Q.k_out) - need_eq;
-          const unsigned long long off = __ldcg(&Q.out_off);
+          const unsigned long long off = __ldcg(&Q.seg_off);
           unsigned long long slot = ~0ull;
           if (lt) {
             const unsigned long long r = bl + __popc(ml & lanemask_lt());
@@ -1219,13 +1226,14 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
   for (unsigned long long i = tid; i < n_sort; i += nth) {
     const unsigned q = __ldcg(p.qids[src] + i);
     p.rank_of[__ldcg(p.vals[src] + i)] =
-        static_cast<int>(i - __ldcg(&p.q[q].out_off));
+        static_cast<int>(i - __ldcg(&p.q[q].seg_off));
   }
   ENG_SYNC();
   for (unsigned long long i = tid; i < n_sort; i += nth) {
     const unsigned idx = __ldcg(p.vals[src] + i);
     const float c = __ldcg(p.ps.cost + idx);
-    p.out_cost[i] = c;
+    const EngineQuery& Q = p.q[__ldcg(p.qids[src] + i)];
+    p.out_cost[__ldcg(&Q.out_off) + (i - __ldcg(&Q.seg_off))] = c;
     if (p.out_nodes) {
       cpg_path_node nd;
       nd.level = __ldcg(p.ps.level + idx);
@@ -1241,6 +1249,413 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
   STAMP(7);
   // the sorted path indices stay in vals[src]; the host learns which buffer
   if (blockIdx.x == 0 && threadIdx.x == 0) p.ctr->sorted_buf = src;
+}
+
+// ------------------------------------------------------------------ one block
+// A query on one block.  Its phases are the grid's (decide, select, promote,
+// closure), but every counter is a shared-memory word, the frontier and the
+// pending pile live in shared memory up to kBlkFront and kBlkPend items (the
+// rest in the block's share of the global piles), and a step is separated
+// from the next by a block barrier alone.  What bounds a round is then the
+// chain of about four dependent loads in grow_path (4.5 us, against 5.4 us
+// when one CTA of the grid engine kept its counters, frontier and pile in
+// global memory); a select pass takes 1.8 us (3.5).  A query of k = 1,000 on
+// the 20,000-pin graph went from 0.32 to 0.19 ms, the first phases of larger
+// ones by about 0.07 ms.
+//
+// A `whole` query is answered to the end and sorted in shared memory; another
+// one is left to the grid launch at the top of a phase with more than
+// solo_stop items pending.  Blocks never wait on one another, so any number
+// of queries run in one ordinary launch, as many at a time as there are SMs.
+constexpr unsigned kBlkPend = 4096, kBlkFront = 1536;
+
+struct BlockMem {
+  Item pend[2][kBlkPend];
+  Item front[2][kBlkFront];
+  unsigned int hist[kSelBins];
+};
+static_assert(sizeof(Item) * 2 * kBlkPend >= 8 * kBlockMaxK, "the sort reuses the pending piles");
+
+// A pile: the first items in shared memory, the others in global memory.
+struct BlkPile {
+  Item* s;
+  Item* g;
+  unsigned scap;
+  unsigned long long gcap;
+  __device__ __forceinline__ Item get(unsigned i) const {
+    return i < scap ? s[i] : load_item(g, i - scap);
+  }
+  __device__ __forceinline__ void put(const EngineParams& p, unsigned i, const Item& it) const {
+    if (i < scap) s[i] = it;
+    else if (i - scap < gcap) g[i - scap] = it;
+    else eng_fail(p, kDevCapacity);
+  }
+};
+
+// This lane's first of n slots of a shared-memory counter (all lanes call).
+__device__ __forceinline__ unsigned blk_reserve(unsigned* ctr, unsigned n) {
+  const int lane = threadIdx.x & 31;
+  unsigned incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  unsigned base = 0;
+  if (lane == 31 && incl) base = atomicAdd(ctr, incl);
+  return __shfl_sync(0xffffffffu, base, 31) + (incl - n);
+}
+
+__device__ __forceinline__ unsigned blk_append(unsigned* ctr, bool on) {
+  const unsigned m = __ballot_sync(0xffffffffu, on);
+  unsigned base = 0;
+  if ((threadIdx.x & 31) == 0 && m) base = atomicAdd(ctr, static_cast<unsigned>(__popc(m)));
+  return __shfl_sync(0xffffffffu, base, 0) + __popc(m & lanemask_lt());
+}
+
+// One pass of the block's radix select: paths base .. base + n_paths when
+// `paths`, then the pending pile; zero costs take part only in a growth
+// phase (mode 1).
+__device__ void blk_hist(const EngineParams& p, unsigned* hist, const EngineQuery& Q,
+                         unsigned long long base, unsigned n_paths, const BlkPile& pend,
+                         unsigned n_pend, int shift, int bits) {
+  const int hi = shift + bits;
+  const unsigned hmask = hi >= 32 ? 0u : ~((1u << hi) - 1u);
+  const unsigned prefix = Q.prefix & hmask;
+  const bool zeros = Q.mode == 1;
+  const unsigned tot = n_paths + n_pend;
+  for (unsigned i0 = threadIdx.x & ~31u; i0 < tot; i0 += blockDim.x) {
+    const unsigned i = i0 + (threadIdx.x & 31);
+    bool on = i < tot;
+    unsigned key = 0;
+    if (on) {
+      const float c = i < n_paths ? __ldcg(p.ps.cost + base + i) : pend.get(i - n_paths).cost;
+      key = float_key(c);
+      on = (zeros || c != 0.0f) && (key & hmask) == prefix;
+    }
+    agg_add_u32(hist, on, (key >> shift) & ((1u << bits) - 1u));
+  }
+}
+
+// Ascending bitonic sort of a[0..n) (padded with ~0 to a power of two by the
+// caller: n2) in shared memory.
+__device__ void blk_sort(unsigned long long* a, unsigned n2) {
+  for (unsigned k = 2; k <= n2; k <<= 1) {
+    for (unsigned j = k >> 1; j > 0; j >>= 1) {
+      for (unsigned t = threadIdx.x; t < n2 / 2; t += blockDim.x) {
+        const unsigned i = 2 * t - (t & (j - 1));  // the pair (i, i + j)
+        const unsigned long long x = a[i], y = a[i + j];
+        if ((x > y) == ((i & k) == 0)) {
+          a[i] = y;
+          a[i + j] = x;
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams p) {
+  extern __shared__ __align__(16) unsigned char blk_raw[];
+  BlockMem& m = *reinterpret_cast<BlockMem*>(blk_raw);
+  __shared__ EngineQuery Q;
+  __shared__ unsigned s_pend[2], s_front[3], s_nz, s_pnz, s_chosen, s_take[2];
+  __shared__ unsigned long long s_base, s_chunk[2];
+  __shared__ int s_go;
+  const int qi = blockIdx.x;
+  const unsigned q = static_cast<unsigned>(qi);
+  const unsigned tid = threadIdx.x, nth = blockDim.x;
+  unsigned long long t_last = 0;
+  if (blockIdx.x == 0 && tid == 0) t_last = gtime();
+  if (tid == 0) {
+    s_stage = 0;
+    Q = p.q[qi];
+    s_pend[0] = s_pend[1] = 0;
+    s_chunk[0] = s_chunk[1] = 0;
+  }
+  for (int i = tid; i < kSelBins; i += nth) m.hist[i] = 0;  // every pick leaves it zero again
+  __syncthreads();
+  const bool whole = Q.whole != 0;
+  // this query's paths: a share of its own, or (several queries, not whole)
+  // chunks of the store the grid launch goes on with
+  const bool own = whole || p.nq == 1;
+  const unsigned long long path_cap = own ? Q.path_base + Q.path_cap : p.ps.cap;
+  Item* const g0 = (whole ? p.pend[0] : p.pend[1]) + Q.pend_base;
+  Item* const g1 = p.pend[1] + Q.pend_base + (whole ? 0 : Q.pend_cap / 2);
+  const unsigned long long pend_gcap = whole ? Q.pend_cap : Q.pend_cap / 2;
+  const unsigned long long front_base = Q.front_base, front_gcap = Q.front_cap;
+  auto pend_pile = [&](int b) { return BlkPile{m.pend[b], b ? g1 : g0, kBlkPend, pend_gcap}; };
+  auto front_pile = [&](int b) {
+    return BlkPile{m.front[b], p.front[b] + front_base, kBlkFront, front_gcap};
+  };
+  if (tid < 32)
+    seed_query(p, qi, Q, [&](bool keep, const Item& it) {
+      const unsigned slot = blk_append(&s_pend[0], keep);
+      if (keep) pend_pile(0).put(p, slot, it);
+    });
+  __syncthreads();
+  STAMP(0);
+
+  int pin = 0, phase = 0, rounds = 0;
+  unsigned n_paths = 0;  // of an `own` query: slots path_base ..
+  for (;; ++phase) {
+    const unsigned n_pend = s_pend[pin];
+    __syncthreads();
+    if (tid == 0) {
+      // (paths in chunks: the final phase, which selects over them, is the
+      // grid's)
+      const bool stay = whole || (n_pend <= p.solo_stop &&
+                                  (own || Q.paths_nz < static_cast<unsigned long long>(Q.k)));
+      s_go = *reinterpret_cast<volatile int*>(&p.ctr->err) == kDevOk && stay &&
+             decide_query(p, Q);
+      s_pend[pin ^ 1] = 0;
+      s_front[0] = s_front[1] = s_front[2] = 0;
+      s_nz = s_pnz = 0;
+    }
+    __syncthreads();
+    if (!s_go) break;
+    STAMP(1);
+    const BlkPile pile = pend_pile(pin), next = pend_pile(pin ^ 1);
+    // select
+    for (int pass = 0; pass < p.sel_passes; ++pass) {
+      const int shift = p.sel_shift[pass], bits = p.sel_bits[pass];
+      blk_hist(p, m.hist, Q, Q.path_base, Q.mode == 2 ? n_paths : 0, pile, n_pend, shift, bits);
+      __syncthreads();
+      select_pick_block<true>(&Q, m.hist, shift, bits, &s_chosen);  // and clears its bins
+      __syncthreads();
+      if (pass == p.sel_passes - 2 && coarse_split(Q, s_chosen)) {
+        __syncthreads();  // every thread has read the query's mode
+        if (tid == 0) {
+          Q.prefix |= (1u << shift) - 1u;
+          Q.coarse = 1;
+        }
+        break;
+      }
+    }
+    __syncthreads();
+    if (tid == 0) set_limit(Q);
+    __syncthreads();
+    STAMP(2);
+    // promote
+    const float lim = Q.lim, tie = Q.tie;
+    unsigned acc_pnz = 0;
+    for (unsigned i0 = tid & ~31u; i0 < n_pend; i0 += nth) {
+      const unsigned i = i0 + (tid & 31);
+      const bool on = i < n_pend;
+      Item it;
+      it.cost = 0.f;
+      if (on) it = pile.get(i);
+      const bool take = on && it.cost <= lim, keep = on && !take;
+      const unsigned a = blk_append(&s_front[0], take);
+      const unsigned b = blk_append(&s_pend[pin ^ 1], keep);
+      if (take) front_pile(0).put(p, a, it);
+      if (keep) next.put(p, b, it);
+      acc_pnz += keep && it.cost != 0.0f;
+    }
+    __syncthreads();
+    STAMP(3);
+    // closure
+    unsigned acc_nz = 0;
+    for (int r = 0;; ++r, ++rounds) {
+      const unsigned n = s_front[r % 3];
+      if (n == 0) break;
+      // (last round's counter, the next round's; nobody reads or adds to it now)
+      if (tid == 0) s_front[(r + 2) % 3] = 0;
+      if (!own) {
+        // n slots in a row; what a chunk leaves over is filled with zero
+        // costs, which no later step counts
+        if (tid == 0) {
+          if (s_chunk[0] + n > s_chunk[1]) {
+            for (unsigned long long x = s_chunk[0]; x < s_chunk[1] && x < p.ps.cap; ++x) {
+              p.ps.cost[x] = 0.f;
+              p.pq[x] = qi;
+            }
+            const unsigned grab = n > 256 ? n : 256;
+            s_chunk[0] = atomicAdd(&p.ctr->paths, static_cast<unsigned long long>(grab));
+            s_chunk[1] = s_chunk[0] + grab;
+          }
+          s_base = s_chunk[0];
+          s_chunk[0] += n;
+        }
+        __syncthreads();
+      }
+      const unsigned long long base = own ? Q.path_base + n_paths : s_base;
+      const BlkPile in = front_pile(r & 1), out = front_pile((r + 1) & 1);
+      for (unsigned i0 = tid & ~31u; i0 < n; i0 += nth) {
+        const unsigned i = i0 + (tid & 31);
+        Item it;
+        it.cost = 0.f;
+        it.parent = -1;
+        it.node = -1;
+        it.j = 0;
+        if (i < n) it = in.get(i);
+        const unsigned long long qp = base + i;
+        const Grown g = grow_path(p, it, i < n, q, qp, path_cap, lim, tie);
+        acc_nz += g.stored && it.cost != 0.0f;
+        acc_pnz += pending_nz(g);
+        unsigned bt = blk_reserve(&s_front[(r + 1) % 3], __popc(g.tm));
+        unsigned bd = blk_reserve(&s_pend[pin ^ 1], __popc(g.dm));
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          const unsigned bit = 1u << k;
+          if (!((g.tm | g.dm) & bit)) continue;
+          const Item c = child_of(g, it, q, qp, k);
+          if (g.tm & bit) out.put(p, bt++, c);
+          else next.put(p, bd++, c);
+        }
+      }
+      n_paths += n;
+      if (__syncthreads_or(tid == 0 && *reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk))
+        break;
+    }
+    acc_nz = __reduce_add_sync(0xffffffffu, acc_nz);
+    acc_pnz = __reduce_add_sync(0xffffffffu, acc_pnz);
+    if ((tid & 31) == 0) {
+      if (acc_nz) atomicAdd(&s_nz, acc_nz);
+      if (acc_pnz) atomicAdd(&s_pnz, acc_pnz);
+    }
+    __syncthreads();
+    if (tid == 0) {
+      if (Q.mode == 2) Q.done = 1;
+      Q.paths_nz += s_nz;
+      Q.pend_n = s_pend[pin ^ 1];
+      Q.pend_nz = s_pnz;
+      Q.pend_next_n = Q.pend_next_nz = 0;
+    }
+    pin ^= 1;
+    __syncthreads();
+    STAMP(4);
+  }
+
+  const unsigned n_pend = s_pend[pin];
+  if (tid == 0) {
+    atomicMax(&p.ctr->res_phase, phase);
+    atomicMax(&p.ctr->phases, phase);
+    atomicAdd(&p.ctr->rounds, rounds);
+  }
+  if (__syncthreads_or(tid == 0 && *reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk))
+    return;
+  if (!whole) {
+    // the rest is the grid's: the pending items join pile 0 and the next
+    // phase is decided there
+    if (tid == 0) {
+      if (own) {
+        p.ctr->paths = n_paths;
+      } else {
+        for (unsigned long long x = s_chunk[0]; x < s_chunk[1] && x < p.ps.cap; ++x) {
+          p.ps.cost[x] = 0.f;
+          p.pq[x] = qi;
+        }
+      }
+      Q.mode = 0;
+      s_base = atomicAdd(&p.ctr->pend_out, static_cast<unsigned long long>(n_pend));
+      p.ctr->stopped = 1;
+    }
+    __syncthreads();
+    const BlkPile left = pend_pile(pin);
+    for (unsigned i = tid; i < n_pend; i += nth) {
+      if (s_base + i < p.pend_cap) p.pend[0][s_base + i] = left.get(i);
+      else eng_fail(p, kDevCapacity);
+    }
+    __syncthreads();
+    if (tid == 0) p.q[qi] = Q;
+    return;
+  }
+
+  // ---- output.  Once K non-zero paths were accepted, the final phase's split
+  // T is the K-th cost of the paths and items then known, and every item up
+  // to T was accepted with its closure: the answer is the paths below T and
+  // as many at T as are missing.  (A closure may produce a child a few ulps
+  // below its parent's T: K or more below T are selected exactly.)  If the
+  // paths ran out before K, every one is reported.
+  const unsigned long long k = static_cast<unsigned long long>(Q.k);
+  const unsigned k_out = static_cast<unsigned>(Q.paths_nz < k ? Q.paths_nz : k);
+  unsigned long long* a = reinterpret_cast<unsigned long long*>(&m.pend[0][0]);
+  const float* cost = p.ps.cost + Q.path_base;
+  unsigned kT = Q.paths_nz >= k ? float_key(Q.t) : 0xffffffffu;
+  for (int attempt = 0; k_out > 0 && attempt < 2; ++attempt) {
+    if (tid == 0) s_take[0] = s_take[1] = 0;
+    __syncthreads();
+    for (unsigned i0 = tid & ~31u; i0 < n_paths; i0 += nth) {
+      const unsigned i = i0 + (tid & 31);
+      const float c = i < n_paths ? __ldcg(cost + i) : 0.f;
+      const unsigned key = float_key(c);
+      const bool lt = c != 0.0f && key < kT;
+      const unsigned slot = blk_append(&s_take[0], lt);
+      if (lt && slot < k_out) a[slot] = (static_cast<unsigned long long>(key) << 32) | i;
+    }
+    __syncthreads();
+    const unsigned below = s_take[0];
+    if (below > k_out) {
+      if (tid == 0) {
+        Q.mode = 3;
+        Q.prefix = 0;
+        Q.krem = k_out;
+      }
+      __syncthreads();
+      for (int pass = 0; pass < p.sel_passes; ++pass) {
+        blk_hist(p, m.hist, Q, Q.path_base, n_paths, pend_pile(0), 0, p.sel_shift[pass],
+                 p.sel_bits[pass]);
+        __syncthreads();
+        select_pick_block<true>(&Q, m.hist, p.sel_shift[pass], p.sel_bits[pass], &s_chosen);
+        __syncthreads();
+      }
+      kT = Q.prefix;
+      __syncthreads();
+      continue;
+    }
+    for (unsigned i0 = tid & ~31u; below < k_out && i0 < n_paths; i0 += nth) {
+      const unsigned i = i0 + (tid & 31);
+      const float c = i < n_paths ? __ldcg(cost + i) : 0.f;
+      const unsigned key = float_key(c);
+      const bool eq = c != 0.0f && key == kT;
+      const unsigned slot = below + blk_append(&s_take[1], eq);
+      if (eq && slot < k_out) a[slot] = (static_cast<unsigned long long>(key) << 32) | i;
+    }
+    break;
+  }
+  unsigned n2 = 1;
+  while (n2 < k_out) n2 <<= 1;
+  for (unsigned i = k_out + tid; i < n2; i += nth) a[i] = ~0ull;
+  __syncthreads();
+  STAMP(5);
+  blk_sort(a, n2);
+  __syncthreads();
+  STAMP(6);
+  for (unsigned i = tid; i < k_out; i += nth)
+    p.out_cost[Q.out_off + i] = key_float(static_cast<unsigned>(a[i] >> 32));
+  if (p.out_nodes) {
+    // paths, their parents' ranks and the sorted path indices
+    for (unsigned i = tid; i < n_paths; i += nth) p.rank_of[Q.path_base + i] = -1;
+    __syncthreads();
+    for (unsigned i = tid; i < k_out; i += nth) {
+      const unsigned idx = static_cast<unsigned>(Q.path_base) + static_cast<unsigned>(a[i]);
+      p.rank_of[idx] = static_cast<int>(i);
+      p.vals[0][Q.out_off + i] = idx;
+    }
+    __syncthreads();
+    for (unsigned i = tid; i < k_out; i += nth) {
+      const unsigned idx = static_cast<unsigned>(Q.path_base) + static_cast<unsigned>(a[i]);
+      cpg_path_node nd;
+      nd.level = __ldcg(p.ps.level + idx);
+      nd.from = __ldcg(p.ps.from + idx);
+      nd.to = __ldcg(p.ps.to + idx);
+      const int par = __ldcg(p.ps.parent + idx);
+      nd.parent = par >= 0 ? __ldcg(p.rank_of + par) : -1;
+      nd.num_children = 0;
+      nd.slack = key_float(static_cast<unsigned>(a[i] >> 32));
+      p.out_nodes[Q.out_off + i] = nd;
+    }
+  }
+  if (tid == 0) {
+    Q.done = 1;
+    Q.mode = 0;
+    Q.k_out = k_out;
+    p.q[qi] = Q;
+    atomicAdd(&p.ctr->blk_paths, static_cast<unsigned long long>(n_paths));
+    atomicAdd(&p.ctr->blk_pend, static_cast<unsigned long long>(n_pend));
+  }
+  STAMP(7);
 }
 
 }  // namespace
@@ -1276,6 +1691,15 @@ int launch_set_queries(EngineQuery* dst, const EngineQuery* src, int nq, void* s
   QueryTable t{};
   for (int i = 0; i < nq; ++i) t.q[i] = src[i];
   set_queries_kernel<<<1, kInlineQueries, 0, static_cast<cudaStream_t>(stream)>>>(dst, t, nq);
+  return cudaGetLastError();
+}
+
+int launch_engine_blocks(const EngineParams& p, void* stream) {
+  const int smem = static_cast<int>(sizeof(BlockMem));
+  cudaError_t e = cudaFuncSetAttribute(engine_block_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return e;
+  engine_block_kernel<<<p.nq, kEngThreads, smem, static_cast<cudaStream_t>(stream)>>>(p);
   return cudaGetLastError();
 }
 
