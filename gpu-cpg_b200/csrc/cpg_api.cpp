@@ -332,7 +332,7 @@ Status upload_graph(cpg_handle* h, int32_t n, int32_t m, const int32_t* adjp,
   CK(ensure(h->d_srcs, nn * 4 + 8), "alloc srcs");
   // suffix tree storage (the deviation array doubles as upload staging)
   CK(ensure(h->d_order, nn * 4), "alloc order");
-  CK(ensure(h->d_queue, (nn + 64) * 4), "alloc queue");
+  CK(ensure(h->d_queue, size_t{128} << sfxt_queue_shift(n)), "alloc queue");
   CK(ensure(h->d_long, nn * 4 + 4), "alloc row list");
   CK(ensure(h->d_dl, nn * 8 + 8), "alloc queue");
   CK(ensure(h->d_lvlp, (nn + 2) * 4), "alloc lvlp");
@@ -562,6 +562,7 @@ SfxtParams sfxt_params(cpg_handle* h, int32_t start_level, bool known = false) {
   p.spin_limit = h->opts.spin_limit ? h->opts.spin_limit : kDefaultSpinLimit;
   p.grid_limit = h->sfxt_grid_limit;
   p.queue = P<int32_t>(h->d_queue);
+  p.queue_shift = sfxt_queue_shift(h->g.n);
   p.long_rows = P<int32_t>(h->d_long);
   p.level_sync = h->opts.sfxt_level_sync == 1;
   p.heap_warps = std::min(std::max(h->opts.sfxt_heap_warps, 0), 16);

@@ -110,6 +110,13 @@ enum DevErr : int {
 // contend for one L2 line.
 constexpr int kMaxClaimSets = 16;
 constexpr int kDefaultClaimSets = 8;
+// The work queue's lines of 32 slots (a power of two): no fewer than every
+// warp of the device can wait on, one each.
+inline int sfxt_queue_shift(int64_t n) {
+  int k = 13;
+  while ((int64_t{32} << k) < n) ++k;
+  return k;
+}
 
 struct SfxtCounters {
   alignas(128) int tail;     // order[] / queue[] append cursor
@@ -187,8 +194,9 @@ struct SfxtParams {
   int32_t known;
   const ChangedGraph* changed;
   int32_t n_changed;
-  // full CSR builds: dataflow work queue (n ints) unless level_sync is set
-  int32_t* queue;
+  // full CSR builds: dataflow work queue unless level_sync is set
+  int32_t* queue;          // 32 << queue_shift ints >= n
+  int32_t queue_shift;
   int32_t* long_rows;      // rows over 64 edges, written unsorted (n ints)
   int32_t level_sync;
   int32_t heap_warps;      // dataflow: warps per CTA that only insert heaps (0: none)

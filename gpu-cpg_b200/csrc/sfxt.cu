@@ -829,9 +829,22 @@ __device__ void heap_insert_lanes(const SfxtParams& p, int v) {
   heap_insert_at<kPublish>(p, v, q, base + (incl - need));
 }
 
+// Where slot s of the work queue lies: consecutive slots on different
+// 128-byte lines.  Every idle warp polls the slot that it claimed, and a
+// store to a line that other warps poll takes 1.2 us to be seen instead of
+// 0.5 (one store to one poll between two SMs, with 30 warps on the line's
+// other words).  With 32 slots a line that wait stood in every level's hop
+// (queued to taken 1.5 us a hop on 20,000 pins, 0.76 now): kernel 0.231 ->
+// 0.180 ms on 20,000 pins, 0.43 -> 0.31 on 100,000, 0.77 -> 0.65 on 300,000,
+// 1.67 -> 1.68 on 1M, whose hops wait for free warps.
+__device__ __forceinline__ int32_t* queue_slot(const SfxtParams& p, int s) {
+  return p.queue + (static_cast<size_t>(s & ((1 << p.queue_shift) - 1)) << 5) +
+         (s >> p.queue_shift);
+}
+
 // The chain-heap phase of a dataflow build (p.heap_phase): after every
 // vertex is built, each lane inserts the heaps of the slots it owns, slots
-// being the work queue from beg on (or a rebuild's level order), where a
+// being the work queue (queued) or the level order from beg on, where a
 // vertex's successor comes before it.  A heap waits
 // only for its successor's, so the waits follow successor chains (about 80
 // hops on the 1M-pin graph) instead of the 200 levels, and no build waits on
@@ -839,13 +852,13 @@ __device__ void heap_insert_lanes(const SfxtParams& p, int v) {
 // successor may be one of them, so the warp inserts, round after round, the
 // lanes whose successor's heap is complete, with one pool reservation per
 // round.  Returns false if a wait ran out.
-__device__ bool heap_phase(const SfxtParams& p, const int32_t* slots, int beg) {
+__device__ bool heap_phase(const SfxtParams& p, bool queued, int beg) {
   const int lane = threadIdx.x & 31;
   const int nw = gridDim.x * (blockDim.x >> 5);
   const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   for (int base = beg + gw * 32; base < p.n; base += nw * 32) {
     const int g = base + lane;
-    int v = g < p.n ? __ldcg(slots + g) : -1;
+    int v = g < p.n ? __ldcg(queued ? queue_slot(p, g) : p.order + g) : -1;
     if (v >= 0 && p.vgraph && !rebuilt(p, v, __ldcg(p.level_of + v))) v = -1;
     const int s = v >= 0 ? __ldcg(p.succ + v) : -1;
     bool pending = v >= 0;
@@ -1097,7 +1110,7 @@ __device__ __forceinline__ int wait_slot(const SfxtParams& p, int s, bool acquir
   int v = -1;
   if ((threadIdx.x & 31) == 0) {
     unsigned int it = 0;
-    const volatile int* q = p.queue + s;
+    const volatile int* q = queue_slot(p, s);
     while ((v = *q) < 0) {
       if (++it > p.spin_limit ||
           ((it & 31) == 0 && *reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk)) {
@@ -1388,7 +1401,7 @@ __device__ int build_vertex_polled(const SfxtParams& p, int v, int rb, int re, D
 // A lane-granular wait for queue slot s (the heap workers).
 __device__ __forceinline__ int wait_slot_lane(const SfxtParams& p, int s) {
   unsigned int it = 0;
-  const volatile int* q = p.queue + s;
+  const volatile int* q = queue_slot(p, s);
   int v;
   while ((v = *q) < 0) {
     if (++it > p.spin_limit ||
@@ -1444,7 +1457,7 @@ __device__ __forceinline__ void queue_push(const SfxtParams& p, bool on, int u) 
   base = __shfl_sync(0xffffffffu, base, leader);
   if (on) {
     const int slot = static_cast<int>(key) * queue_seg(p) + base + __popc(m & lanemask_lt());
-    *reinterpret_cast<volatile int*>(p.queue + slot) = u;
+    *reinterpret_cast<volatile int*>(queue_slot(p, slot)) = u;
   }
 }
 
@@ -1496,7 +1509,7 @@ __device__ __forceinline__ void dataflow_push(const SfxtParams& p, int v, int ib
     slot0 = __shfl_sync(0xffffffffu, slot0, 0);
 #pragma unroll
     for (int c = 0; c < kC; ++c)
-      if ((ready >> c) & 1u) *reinterpret_cast<volatile int*>(p.queue + slot0 + mine[c]) = u[c];
+      if ((ready >> c) & 1u) *reinterpret_cast<volatile int*>(queue_slot(p, slot0 + mine[c])) = u[c];
   }
 }
 
@@ -1612,7 +1625,7 @@ sfxt_dataflow_kernel(SfxtParams p) {
     p.order[v] = 0;  // build-published flags until the final level sort
     p.dl[v] = ~0ull;  // (dist, level) not published yet
   }
-  for (int i = tid; i < kSfxtQueues * queue_seg(p); i += nth) p.queue[i] = -1;
+  for (int i = tid; i < 32 << p.queue_shift; i += nth) p.queue[i] = -1;
   for (int i = tid; i < p.n + 2; i += nth) p.lvlp[i] = 0;
   if (!grid_sync(&p.ctr->bar, &p.ctr->err, p.spin_limit)) return;
   // the sinks start the queue
@@ -1724,7 +1737,7 @@ sfxt_dataflow_kernel(SfxtParams p) {
       *reinterpret_cast<volatile int*>(&p.ctr->sort_ready) = 1;
     }
   }
-  if (hp) ok = heap_phase(p, p.queue, 0) && ok;
+  if (hp) ok = heap_phase(p, true, 0) && ok;
   // scatter this block's vertices by level: one reservation per (block,
   // level) on the level's cursor (deps[], all zero once every vertex was
   // queued), then a shared-memory cursor per level
@@ -1903,7 +1916,7 @@ sfxt_known_kernel(SfxtParams p) {
   if (!known_walk<true>(p, beg, p.n, gw, nw, !hp, chunk)) return;
   if (hp) {
     if (!grid_sync(&p.ctr->bar, &p.ctr->err, p.spin_limit)) return;
-    heap_phase(p, p.order, beg);
+    heap_phase(p, false, beg);
   }
 }
 
