@@ -1160,6 +1160,143 @@ __device__ __forceinline__ void publish_dl(const SfxtParams& p, int v, int lvl, 
         static_cast<unsigned>(best);
 }
 
+// Early-push build of a row of at most 32 C edges: the whole row in registers,
+// C words a lane.  best, s, cnt, lmax and top are build_vertex_polled's; false
+// if a wait ran out (warp-uniform).  One copy per C: a warp issues a dependent
+// instruction every few cycles at best, and rows of one word a lane (80 % of
+// them at mean degree 20) that ran through eight words' steps spent more time
+// on those than on their loads (kernel 1.68 -> 1.59 ms on the 1M-pin graph, 0.65 ->
+// 0.62 on 300,000 pins).
+template <int C>
+__device__ __forceinline__ bool build_row_polled(const SfxtParams& p, int v, int rb, int re,
+                                                 const DevEdge& ed0, unsigned long long dl0,
+                                                 int& best, int& s, int& cnt, int& lmax,
+                                                 DevSidetrack& top) {
+  const int lane = threadIdx.x & 31;
+  constexpr unsigned long long kNone = ~0ull;
+  DevEdge ed[C];
+  int dh[C];
+  ed[0] = ed0;  // loaded before the push (dl0: its head's word, or ~0)
+#pragma unroll
+  for (int c = 1; c < C; ++c) {
+    const int e = rb + c * 32 + lane;
+    ed[c].head = -1;
+    ed[c].w = 0.f;
+    if (e < re) ed[c] = p.edges[e];
+  }
+  unsigned pending = 0;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    dh[c] = INT_MAX;
+    if (ed[c].head >= 0) {
+      // a published word never changes: one read before the push stands
+      const unsigned long long x = c == 0 && dl0 != kNone ? dl0 : ld_dl(p, ed[c].head);
+      if (x == kNone) {
+        pending |= 1u << c;
+      } else {
+        dh[c] = static_cast<int>(x & 0xffffffffu);
+        lmax = max(lmax, static_cast<int>(x >> 32));
+      }
+    }
+  }
+  unsigned int it = 0;
+  while (__any_sync(0xffffffffu, pending != 0)) {
+    // the lanes may read err differently: decide for the whole warp
+    ++it;
+    const bool bail = __any_sync(0xffffffffu, it > p.spin_limit ||
+                                 ((it & 31) == 0 &&
+                                  *reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk));
+    if (bail) {
+      if (lane == 0) atomicCAS(&p.ctr->err, kDevOk, kDevTimeout);
+      return false;
+    }
+    __nanosleep(32);
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      if (pending & (1u << c)) {
+        const unsigned long long x = ld_dl(p, ed[c].head);
+        if (x != kNone) {
+          dh[c] = static_cast<int>(x & 0xffffffffu);
+          lmax = max(lmax, static_cast<int>(x >> 32));
+          pending &= ~(1u << c);
+        }
+      }
+    }
+  }
+  const int lvl = warp_max_i(lmax) + 1;
+  if (lvl == 0) {
+    best = 0;  // a sink
+    publish_dl(p, v, lvl, best);
+  } else {
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      if (ed[c].head >= 0) best = min(best, cand_dist(dh[c], ed[c].w));
+    best = warp_min_i(best);
+    publish_dl(p, v, lvl, best);
+    int nt = 0;  // this lane's tied heads
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      if (ed[c].head >= 0 && cand_dist(dh[c], ed[c].w) == best) {
+        s = max(s, ed[c].head);
+        ++nt;
+      }
+    if (p.orig_id && __reduce_add_sync(0xffffffffu, nt) > 1) {
+      unsigned long long k = 0;
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+        if (ed[c].head >= 0 && cand_dist(dh[c], ed[c].w) == best) {
+          const unsigned long long x = succ_word(p, ed[c].head);
+          k = x > k ? x : k;
+        }
+      s = static_cast<int>(group_max_u64<32>(k) & 0xffffffffu);
+    } else {
+      s = warp_max_i(s);
+    }
+  }
+  if constexpr (C == 1) {
+    const bool valid = ed[0].head >= 0 && ed[0].head != s && dh[0] != INT_MAX;
+    DevSidetrack rec;
+    rec.head = ed[0].head;
+    rec.w = ed[0].w;
+    rec.dist_head = dh[0];
+    rec.key = deviation_key(dh[0], best, ed[0].w);
+    cnt = write_short_row(p, rb, valid, rec, top);
+  } else if constexpr (C == 2) {
+    DevSidetrack r[2];
+    bool v[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      v[c] = ed[c].head >= 0 && ed[c].head != s && dh[c] != INT_MAX;
+      r[c].head = ed[c].head;
+      r[c].w = ed[c].w;
+      r[c].dist_head = dh[c];
+      r[c].key = deviation_key(dh[c], best, ed[c].w);
+    }
+    cnt = write_row64(p, rb, v[0], r[0], v[1], r[1], top);
+  } else {
+    BestDev bd = best_none();
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      if (rb + c * 32 >= re) break;
+      const bool valid = ed[c].head >= 0 && ed[c].head != s && dh[c] != INT_MAX;
+      const unsigned bal = __ballot_sync(0xffffffffu, valid);
+      if (valid) {
+        DevSidetrack rec;
+        rec.head = ed[c].head;
+        rec.w = ed[c].w;
+        rec.dist_head = dh[c];
+        rec.key = deviation_key(dh[c], best, ed[c].w);
+        p.dev[rb + cnt + __popc(bal & lanemask_lt())] = rec;
+        best_take(bd, true, rec, c * 32 + lane);
+      }
+      cnt += __popc(bal);
+    }
+    top = best_reduce(bd);
+  }
+  lmax = lvl;
+  return true;
+}
+
 __device__ int build_vertex_polled(const SfxtParams& p, int v, int rb, int re, DevEdge ed0,
                                    unsigned long long dl0) {
   const int lane = threadIdx.x & 31;
@@ -1170,127 +1307,12 @@ __device__ int build_vertex_polled(const SfxtParams& p, int v, int rb, int re, D
   DevSidetrack top;  // the cheapest deviation (lane 0's copy is used)
   top.head = -1;
   constexpr unsigned long long kNone = ~0ull;
-  if (re - rb <= kRegChunks * 32) {
-    DevEdge ed[kRegChunks];
-    int dh[kRegChunks];
-    ed[0] = ed0;  // loaded before the push (dl0: its head's word, or ~0)
-#pragma unroll
-    for (int c = 1; c < kRegChunks; ++c) {
-      const int e = rb + c * 32 + lane;
-      ed[c].head = -1;
-      ed[c].w = 0.f;
-      if (e < re) ed[c] = p.edges[e];
-    }
-    unsigned pending = 0;
-#pragma unroll
-    for (int c = 0; c < kRegChunks; ++c) {
-      dh[c] = INT_MAX;
-      if (ed[c].head >= 0) {
-        // a published word never changes: one read before the push stands
-        const unsigned long long x = c == 0 && dl0 != kNone ? dl0 : ld_dl(p, ed[c].head);
-        if (x == kNone) {
-          pending |= 1u << c;
-        } else {
-          dh[c] = static_cast<int>(x & 0xffffffffu);
-          lmax = max(lmax, static_cast<int>(x >> 32));
-        }
-      }
-    }
-    unsigned int it = 0;
-    while (__any_sync(0xffffffffu, pending != 0)) {
-      // the lanes may read err differently: decide for the whole warp
-      ++it;
-      const bool bail = __any_sync(0xffffffffu, it > p.spin_limit ||
-                                   ((it & 31) == 0 &&
-                                    *reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk));
-      if (bail) {
-        if (lane == 0) atomicCAS(&p.ctr->err, kDevOk, kDevTimeout);
-        return -1;
-      }
-      __nanosleep(32);
-#pragma unroll
-      for (int c = 0; c < kRegChunks; ++c) {
-        if (pending & (1u << c)) {
-          const unsigned long long x = ld_dl(p, ed[c].head);
-          if (x != kNone) {
-            dh[c] = static_cast<int>(x & 0xffffffffu);
-            lmax = max(lmax, static_cast<int>(x >> 32));
-            pending &= ~(1u << c);
-          }
-        }
-      }
-    }
-    const int lvl = warp_max_i(lmax) + 1;
-    if (lvl == 0) {
-      best = 0;  // a sink
-      publish_dl(p, v, lvl, best);
-    } else {
-#pragma unroll
-      for (int c = 0; c < kRegChunks; ++c)
-        if (ed[c].head >= 0) best = min(best, cand_dist(dh[c], ed[c].w));
-      best = warp_min_i(best);
-      publish_dl(p, v, lvl, best);
-      int nt = 0;  // this lane's tied heads
-#pragma unroll
-      for (int c = 0; c < kRegChunks; ++c)
-        if (ed[c].head >= 0 && cand_dist(dh[c], ed[c].w) == best) {
-          s = max(s, ed[c].head);
-          ++nt;
-        }
-      if (p.orig_id && __reduce_add_sync(0xffffffffu, nt) > 1) {
-        unsigned long long k = 0;
-#pragma unroll
-        for (int c = 0; c < kRegChunks; ++c)
-          if (ed[c].head >= 0 && cand_dist(dh[c], ed[c].w) == best) {
-            const unsigned long long x = succ_word(p, ed[c].head);
-            k = x > k ? x : k;
-          }
-        s = static_cast<int>(group_max_u64<32>(k) & 0xffffffffu);
-      } else {
-        s = warp_max_i(s);
-      }
-    }
-    if (re - rb <= 32) {
-      const bool valid = ed[0].head >= 0 && ed[0].head != s && dh[0] != INT_MAX;
-      DevSidetrack rec;
-      rec.head = ed[0].head;
-      rec.w = ed[0].w;
-      rec.dist_head = dh[0];
-      rec.key = deviation_key(dh[0], best, ed[0].w);
-      cnt = write_short_row(p, rb, valid, rec, top);
-    } else if (re - rb <= 64) {
-      DevSidetrack r[2];
-      bool v[2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        v[c] = ed[c].head >= 0 && ed[c].head != s && dh[c] != INT_MAX;
-        r[c].head = ed[c].head;
-        r[c].w = ed[c].w;
-        r[c].dist_head = dh[c];
-        r[c].key = deviation_key(dh[c], best, ed[c].w);
-      }
-      cnt = write_row64(p, rb, v[0], r[0], v[1], r[1], top);
-    } else {
-      BestDev bd = best_none();
-#pragma unroll
-      for (int c = 0; c < kRegChunks; ++c) {
-        if (rb + c * 32 >= re) break;
-        const bool valid = ed[c].head >= 0 && ed[c].head != s && dh[c] != INT_MAX;
-        const unsigned bal = __ballot_sync(0xffffffffu, valid);
-        if (valid) {
-          DevSidetrack rec;
-          rec.head = ed[c].head;
-          rec.w = ed[c].w;
-          rec.dist_head = dh[c];
-          rec.key = deviation_key(dh[c], best, ed[c].w);
-          p.dev[rb + cnt + __popc(bal & lanemask_lt())] = rec;
-          best_take(bd, true, rec, c * 32 + lane);
-        }
-        cnt += __popc(bal);
-      }
-      top = best_reduce(bd);
-    }
-    lmax = lvl;
+  if (re - rb <= 32) {
+    if (!build_row_polled<1>(p, v, rb, re, ed0, dl0, best, s, cnt, lmax, top)) return -1;
+  } else if (re - rb <= 64) {
+    if (!build_row_polled<2>(p, v, rb, re, ed0, dl0, best, s, cnt, lmax, top)) return -1;
+  } else if (re - rb <= kRegChunks * 32) {
+    if (!build_row_polled<kRegChunks>(p, v, rb, re, ed0, dl0, best, s, cnt, lmax, top)) return -1;
   } else {
     // Long rows (a super-source's, say), eight chunks of 32 edges per pass
     // with every load of a pass issued before any is used.  Pass 1 waits for

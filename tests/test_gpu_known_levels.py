@@ -115,3 +115,40 @@ def test_edge_id_out_of_range_changes_nothing():
         g.report_paths(500)
         assert np.array_equal(g.get_slacks(500), before)
         assert np.array_equal(g.get_csr()[2], w)
+
+
+@pytest.mark.parametrize("heap_mode", [1, 2])
+@pytest.mark.parametrize("deg", [1, 31, 32, 33, 63, 64, 65, 128, 129, 255, 256, 257, 700])
+def test_rows_at_the_edges_of_the_register_words(deg, heap_mode):
+    """Full and known-level builds of rows of exactly `deg` edges, some with a
+    parallel path of equal cost (ties), in either heap regime."""
+    rng = np.random.default_rng(deg)
+    width, levels = max(deg, 5), 4
+    n = levels * width + 2
+    src, dst = [], []
+    for lv in range(levels - 1):
+        for i in rng.choice(width, 9, replace=width < 9):
+            heads = rng.choice(width, deg, replace=False)
+            src += [lv * width + int(i)] * deg
+            dst += ((lv + 1) * width + heads).tolist()
+    pairs = np.unique(np.stack([src, dst], 1), axis=0)
+    tails = np.setdiff1d(pairs[:, 1], pairs[:, 0])
+    heads = np.setdiff1d(pairs[:, 0], pairs[:, 1])
+    pairs = np.concatenate([pairs, np.stack([tails, np.full(tails.size, n - 1)], 1),
+                            np.stack([np.full(heads.size, n - 2), heads], 1)])
+    src, dst = pairs[:, 0].astype(np.int32), pairs[:, 1].astype(np.int32)
+    w = rng.integers(1, 6, src.size).astype(np.float32)
+    adjp, adj, w = _csr(n, src, dst, w)
+    tail = np.repeat(np.arange(n, dtype=np.int32), np.diff(adjp))
+    with cpg_b200.CpGen(division=cpg_b200.DIV_IEEE, sfxt_heap_mode=heap_mode) as g:
+        g.load_csr(n, adjp, adj, w)
+        for step in range(2):
+            og = oracle.OracleGraph.from_edges(n, tail, adj, w)
+            for a, b in zip(g.get_sfxt(), og.sfxt()):
+                np.testing.assert_array_equal(a, b)
+            want = og.closure_topk(1500)[0]["slack"]
+            g.report_paths(1500)
+            assert np.array_equal(g.get_slacks(1500).view(np.uint32), want.view(np.uint32))
+            e = rng.choice(adj.size, 1 + adj.size // 3, replace=False).astype(np.int32)
+            w[e] = rng.integers(1, 6, e.size).astype(np.float32)
+            g.update_delays(e, w[e])
