@@ -1538,11 +1538,11 @@ __device__ __forceinline__ void dataflow_push(const SfxtParams& p, int v, int ib
 // One taken queue slot of the dataflow build: v's Kahn push and build (in
 // either order), then its chain-heap insert unless the heap phase (kHp) or
 // the heap workers do it.  False when a wait ran out (warp-uniform).
-template <bool kHp>
+template <bool kHp, bool kAb>
 __device__ __forceinline__ bool dataflow_slot(const SfxtParams& p, int v, int heap_warps,
                                               unsigned long long* chunk, int& max_lvl) {
   const int lane = threadIdx.x & 31;
-  if (p.early_push) {
+  if (!kAb || p.early_push) {
     // the tails learn of v before it is built; they wait on its word.
     // Graphs big enough for the heap phase keep a backlog of queued vertices
     // through most of the wave, so the warps' round trips count: the build's
@@ -1600,7 +1600,7 @@ __device__ __forceinline__ bool dataflow_slot(const SfxtParams& p, int v, int he
 // still building waits for nobody: any idle warp of the set takes it.  The S
 // counters spread the claims (one atomic per vertex).  Static slots (S = 0):
 // build warp bw serves queue bw % kSfxtQueues, taking every nwq-th slot.
-template <bool kHp>
+template <bool kHp, bool kAb>
 __device__ __forceinline__ void dataflow_build_warp(const SfxtParams& p, int wib, int build_warps,
                                                     int heap_warps, unsigned long long* chunk,
                                                     int& max_lvl) {
@@ -1614,7 +1614,7 @@ __device__ __forceinline__ void dataflow_build_warp(const SfxtParams& p, int wib
   const int seg0 = q * queue_seg(p);
   for (int k = bw / kSfxtQueues;; k += nwq) {
     int slot;
-    if (S > 0) {
+    if (!kAb || S > 0) {
       int t = 0;
       if (lane == 0) t = atomicAdd(&p.ctr->claim[q][0], 1);
       t = __shfl_sync(0xffffffffu, t, 0);
@@ -1624,13 +1624,28 @@ __device__ __forceinline__ void dataflow_build_warp(const SfxtParams& p, int wib
       if (k >= cnt) break;
       slot = seg0 + k;
     }
-    const int v = wait_slot(p, slot, !p.early_push);
-    if (v < 0 || !dataflow_slot<kHp>(p, v, heap_warps, chunk, max_lvl)) break;
+    const int v = wait_slot(p, slot, kAb && !p.early_push);
+    if (v < 0 || !dataflow_slot<kHp, kAb>(p, v, heap_warps, chunk, max_lvl)) break;
   }
 }
 
+// The heap phase pays once the build warps have over ~128 vertices each
+// (measured: it loses 0.25-0.45 ms from 200,000 to 400,000 vertices, where its
+// chain of successor heaps is not hidden, and wins 0.2-0.35 ms at 1,000,000).
+__host__ __device__ inline bool use_heap_phase(const SfxtParams& p, int grid, int build_warps) {
+  return p.heap_phase == 2 || (p.heap_phase == 1 && p.n >= 128 * grid * build_warps);
+}
+
+// kMode: 0 chain heaps inserted by the building warps, 1 in the heap phase,
+// both with early push and claimed slots; 2 any A/B option set.  A kernel per
+// regime, so that each holds one copy of the loop: with all copies in one
+// kernel the warps, each at another place of it, waited for instructions
+// (0.62 -> 0.59 ms on 300,000 pins, 0.76 -> 0.72 on 400,000, 1.59 -> 1.55 on
+// 1M).
+template <int kMode>
 __global__ void __launch_bounds__(kSfxtThreads)
 sfxt_dataflow_kernel(SfxtParams p) {
+  constexpr bool kAb = kMode == 2;
   __shared__ int s_hist[kSfxtThreads];
   const int lane = threadIdx.x & 31;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1665,20 +1680,16 @@ sfxt_dataflow_kernel(SfxtParams p) {
   unsigned long long* chunk = s_chunk[wib];
   if (lane == 0) chunk[0] = chunk[1] = 0;
   __syncwarp();
-  const int heap_warps = p.heap_warps;  // 0: the build warp inserts the heap itself
+  const int heap_warps = kAb ? p.heap_warps : 0;  // 0: the build warp inserts the heap itself
   const int build_warps = kSfxtThreads / 32 - heap_warps;
-  // The heap phase pays once the build warps have over ~128 vertices each
-  // (measured: it loses 0.25-0.45 ms from 200,000 to 400,000 vertices,
-  // where its chain of successor heaps is not hidden, and wins 0.2-0.35 ms
-  // at 1,000,000)
-  const bool hp = p.heap_phase == 2 ||
-                  (p.heap_phase == 1 && p.n >= 128 * static_cast<int>(gridDim.x) * build_warps);
-  if (wib < build_warps) {
-    // one copy of the loop per regime, each compiled for its own order
+  const bool hp = kAb ? use_heap_phase(p, gridDim.x, build_warps) : kMode == 1;
+  if (!kAb) {
+    dataflow_build_warp<kMode == 1, false>(p, wib, build_warps, 0, chunk, max_lvl);
+  } else if (wib < build_warps) {
     if (hp)
-      dataflow_build_warp<true>(p, wib, build_warps, heap_warps, chunk, max_lvl);
+      dataflow_build_warp<true, true>(p, wib, build_warps, heap_warps, chunk, max_lvl);
     else
-      dataflow_build_warp<false>(p, wib, build_warps, heap_warps, chunk, max_lvl);
+      dataflow_build_warp<false, true>(p, wib, build_warps, heap_warps, chunk, max_lvl);
   } else {
     const int nhl = gridDim.x * heap_warps * 32;
     const int seg = queue_seg(p);
@@ -2061,8 +2072,15 @@ int launch_sfxt(const SfxtParams& p, int device, void* stream, int* grid_out,
   const bool dataflow = !bvss && p.start_level == 0 && !p.level_sync;
   void* kern = p.known    ? reinterpret_cast<void*>(sfxt_known_kernel)
                : bvss     ? reinterpret_cast<void*>(sfxt_persistent_kernel<true>)
-               : dataflow ? reinterpret_cast<void*>(sfxt_dataflow_kernel)
+               : dataflow ? reinterpret_cast<void*>(sfxt_dataflow_kernel<2>)
                           : reinterpret_cast<void*>(sfxt_persistent_kernel<false>);
+  if (dataflow && !p.known && p.early_push && p.claim_sets > 0 && p.heap_warps == 0) {
+    // (one CTA of 1,024 threads and 64 registers a thread fits an SM)
+    const int ctas = p.grid_limit > 0 && p.grid_limit < sms ? p.grid_limit : sms;
+    kern = use_heap_phase(p, ctas, kSfxtThreads / 32)
+               ? reinterpret_cast<void*>(sfxt_dataflow_kernel<1>)
+               : reinterpret_cast<void*>(sfxt_dataflow_kernel<0>);
+  }
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSfxtThreads, 0);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
