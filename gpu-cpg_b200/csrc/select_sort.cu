@@ -374,72 +374,398 @@ namespace cpg {
 
 namespace {
 
-__global__ void keys_to_costs_kernel(const unsigned int* keys, unsigned long long n,
-                                     float* out) {
+// ---- the standalone top-K: the k smallest non-zero values, nothing else.
+// Keys are taken relative to the least one, so the digits start at the
+// highest bit in which the values differ: costs of a few delay units' range
+// share their exponent, and an 11-bit digit of the raw key would put them in
+// a handful of bins.  Five launches read the values (range, up to three
+// digits, compaction; each reserves output once per block), the survivors are
+// sorted alone without indices, and the host waits once, at the end.  8 M
+// values, k = 200,000: 1.1-1.5 -> 0.20 ms (a count, three 11-bit digits of the
+// raw keys, an output reservation per warp and a one-block scan per sort pass
+// before; 0.2-0.5 ms of it cudaMalloc and cudaFree).
+constexpr int kTopkThreads = 1024;
+constexpr int kTopkBins = 2048;
+
+struct TopkState {
+  unsigned int nz;        // non-zero values
+  unsigned int key_max;   // largest key, and ~ the smallest (zero at the start)
+  unsigned int inv_min;
+  unsigned int prefix;    // decided high bits of the k-th relative key
+  unsigned int k_rem;     // its rank inside the prefix
+  unsigned int bits_left; // bits below the prefix
+  unsigned int ticket;    // blocks done with a digit
+  unsigned int n_lt, n_eq;
+};
+static_assert(sizeof(TopkState) <= kTopkStateWords * 4, "state outgrew its scratch");
+
+__device__ __forceinline__ unsigned topk_k(const TopkState* st, unsigned long long k) {
+  const unsigned nz = __ldcg(&st->nz);
+  return k < nz ? static_cast<unsigned>(k) : nz;
+}
+
+// f(value) for every value, four to a load where the address allows it
+template <typename F>
+__device__ __forceinline__ void topk_each(const float* a, unsigned long long n, F&& f) {
+  const unsigned long long tid =
+      static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const unsigned long long nth = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
+  // values before the first 16-byte boundary, whole vectors, the rest
+  unsigned long long head = ((16 - (reinterpret_cast<unsigned long long>(a) & 15)) & 15) / 4;
+  if (head > n) head = n;
+  const unsigned long long nv = (n - head) / 4;
+  const float4* v = reinterpret_cast<const float4*>(a + head);
+  for (unsigned long long i = tid; i < nv; i += nth) {
+    const float4 x = __ldcg(v + i);
+    f(x.x);
+    f(x.y);
+    f(x.z);
+    f(x.w);
+  }
+  if (tid < head) f(__ldcg(a + tid));
+  const unsigned long long tail = head + 4 * nv + tid;
+  if (tail < n) f(__ldcg(a + tail));
+}
+
+__global__ void __launch_bounds__(kTopkThreads)
+topk_range_kernel(const float* a, unsigned long long n, TopkState* st) {
+  unsigned nz = 0, mx = 0, inv = 0;
+  topk_each(a, n, [&](float x) {
+    if (x != 0.0f) {
+      const unsigned key = float_key(x);
+      ++nz;
+      mx = max(mx, key);
+      inv = max(inv, ~key);
+    }
+  });
+  __shared__ unsigned s[3];
+  if (threadIdx.x < 3) s[threadIdx.x] = 0;
+  __syncthreads();
+  nz = __reduce_add_sync(0xffffffffu, nz);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  inv = __reduce_max_sync(0xffffffffu, inv);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&s[0], nz);
+    atomicMax(&s[1], mx);
+    atomicMax(&s[2], inv);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && s[0]) {
+    atomicAdd(&st->nz, s[0]);
+    atomicMax(&st->key_max, s[1]);
+    atomicMax(&st->inv_min, s[2]);
+  }
+}
+
+// One digit of the select: up to 11 bits below the decided prefix.  The last
+// block to add its histogram finds the digit of the k-th key and leaves the
+// histogram zero.
+__global__ void __launch_bounds__(kTopkThreads)
+topk_digit_kernel(const float* a, unsigned long long n, unsigned long long k, TopkState* st,
+                  unsigned int* hist, bool first) {
+  __shared__ unsigned int sh[kTopkBins];
+  __shared__ unsigned int s_warp[32];
+  __shared__ bool s_last;
+  const unsigned kk = topk_k(st, k);
+  const unsigned lo = ~__ldcg(&st->inv_min), range = __ldcg(&st->key_max) - lo;
+  const int hi = kk == 0 ? 0
+               : first   ? 32 - __clz(range)
+                         : static_cast<int>(__ldcg(&st->bits_left));
+  if (hi == 0) return;  // decided (or nothing to select), for every block
+  const int shift = hi > 11 ? hi - 11 : 0, bins = 1 << (hi - shift);
+  const unsigned prefix = first ? 0u : __ldcg(&st->prefix);
+  const unsigned krem = first ? kk : __ldcg(&st->k_rem);
+  for (int i = threadIdx.x; i < kTopkBins; i += blockDim.x) sh[i] = 0;
+  __syncthreads();
+  topk_each(a, n, [&](float x) {
+    if (x != 0.0f) {
+      const unsigned rel = float_key(x) - lo;
+      if (hi >= 32 || (rel >> hi) == (prefix >> hi))
+        atomicAdd(&sh[(rel >> shift) & (bins - 1)], 1u);
+    }
+  });
+  __syncthreads();
+  for (int i = threadIdx.x; i < bins; i += blockDim.x)
+    if (sh[i]) atomicAdd(&hist[i], sh[i]);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&st->ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // two bins a thread, a block scan, and the thread whose bins hold rank krem
+  const int b0 = 2 * static_cast<int>(threadIdx.x);
+  const unsigned h0 = b0 < bins ? __ldcg(hist + b0) : 0u;
+  const unsigned h1 = b0 + 1 < bins ? __ldcg(hist + b0 + 1) : 0u;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned incl = h0 + h1;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_warp[wid] = incl;
+  __syncthreads();
+  if (wid == 0) {
+    unsigned w = s_warp[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    s_warp[lane] = w;
+  }
+  __syncthreads();
+  if (wid > 0) incl += s_warp[wid - 1];
+  const unsigned excl = incl - h0 - h1;
+  if (excl < krem && krem <= incl) {
+    const bool second = krem - excl > h0;
+    st->prefix = prefix | (static_cast<unsigned>(b0 + second) << shift);
+    st->k_rem = krem - excl - (second ? h0 : 0u);
+    st->bits_left = static_cast<unsigned>(shift);
+    st->ticket = 0;
+  }
+  if (b0 < bins) hist[b0] = 0;
+  if (b0 + 1 < bins) hist[b0 + 1] = 0;
+}
+
+// Relative keys below the k-th, and as many equal to it as are missing.
+__global__ void __launch_bounds__(kTopkThreads)
+topk_compact_kernel(const float* a, unsigned long long n, unsigned long long k, TopkState* st,
+                    unsigned int* keys) {
+  __shared__ unsigned s_w[32];  // per warp: below
+  __shared__ unsigned s_e[32];  // ... and equal
+  __shared__ unsigned s_base[2];
+  const unsigned kk = topk_k(st, k);
+  if (kk == 0) return;
+  const unsigned lo = ~__ldcg(&st->inv_min), range = __ldcg(&st->key_max) - lo;
+  const unsigned kth = range ? __ldcg(&st->prefix) : 0u;
+  const unsigned need_eq = range ? __ldcg(&st->k_rem) : kk;
+  const unsigned n_lt = kk - need_eq;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  constexpr int kPer = 8;
+  const unsigned long long tile = static_cast<unsigned long long>(blockDim.x) * kPer;
+  for (unsigned long long t0 = blockIdx.x * tile; t0 < n; t0 += gridDim.x * tile) {
+    unsigned rel[kPer], lt = 0, eq = 0;
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      const unsigned long long i = t0 + c * blockDim.x + threadIdx.x;
+      const float x = i < n ? __ldcg(a + i) : 0.0f;
+      rel[c] = float_key(x) - lo;
+      if (x != 0.0f) {
+        if (rel[c] < kth) lt |= 1u << c;
+        else if (rel[c] == kth) eq |= 1u << c;
+      }
+    }
+    unsigned li = __popc(lt), ei = __popc(eq);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, li, o), z = __shfl_up_sync(0xffffffffu, ei, o);
+      if (lane >= o) {
+        li += y;
+        ei += z;
+      }
+    }
+    if (lane == 31) {
+      s_w[wid] = li;
+      s_e[wid] = ei;
+    }
+    __syncthreads();
+    if (wid == 0) {
+      unsigned w = s_w[lane], e = s_e[lane];
+      const unsigned w0 = w, e0 = e;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, w, o), z = __shfl_up_sync(0xffffffffu, e, o);
+        if (lane >= o) {
+          w += y;
+          e += z;
+        }
+      }
+      s_w[lane] = w - w0;
+      s_e[lane] = e - e0;
+      if (lane == 31) {
+        s_base[0] = w ? atomicAdd(&st->n_lt, w) : 0u;
+        s_base[1] = e ? atomicAdd(&st->n_eq, e) : 0u;
+      }
+    }
+    __syncthreads();
+    unsigned sl = s_base[0] + s_w[wid] + li - __popc(lt);
+    unsigned se = s_base[1] + s_e[wid] + ei - __popc(eq);
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      if ((lt >> c) & 1u) {
+        if (sl < n_lt) keys[sl] = rel[c];
+        ++sl;
+      }
+      if ((eq >> c) & 1u) {
+        if (se < need_eq) keys[n_lt + se] = rel[c];
+        ++se;
+      }
+    }
+    __syncthreads();  // the shared words are reused
+  }
+}
+
+// ---- LSD sort of the survivors, 8 bits a pass over the bits of the k-th
+// key; a pass above them ends at once
+__device__ __forceinline__ int topk_passes(const TopkState* st) {
+  const unsigned lo = ~__ldcg(&st->inv_min);
+  const unsigned kth = __ldcg(&st->key_max) == lo ? 0u : __ldcg(&st->prefix);
+  return (32 - __clz(kth) + 7) / 8;
+}
+
+__global__ void topk_sort_hist_kernel(const unsigned int* keys, unsigned long long k,
+                                      const TopkState* st, int pass, unsigned int* hist,
+                                      int nblocks) {
+  __shared__ unsigned int sh[256];
+  if (pass >= topk_passes(st)) return;
+  const unsigned kk = topk_k(st, k);
+  sh[threadIdx.x] = 0;
+  __syncthreads();
+  const unsigned long long base = static_cast<unsigned long long>(blockIdx.x) * kSortTile;
+#pragma unroll
+  for (int t = 0; t < kSortItems; ++t) {
+    const unsigned long long i = base + t * kSortThreads + threadIdx.x;
+    if (i < kk) atomicAdd(&sh[(keys[i] >> (8 * pass)) & 255u], 1u);
+  }
+  __syncthreads();
+  hist[static_cast<size_t>(threadIdx.x) * nblocks + blockIdx.x] = sh[threadIdx.x];
+}
+
+// A warp per digit: exclusive scan over the tiles, the digit's total last.
+__global__ void topk_sort_rows_kernel(const TopkState* st, int pass, unsigned int* hist,
+                                      int nblocks, unsigned int* totals) {
+  if (pass >= topk_passes(st)) return;
+  const int d = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (d >= 256) return;
+  unsigned int* row = hist + static_cast<size_t>(d) * nblocks;
+  unsigned carry = 0;
+  for (int b0 = 0; b0 < nblocks; b0 += 32) {
+    const int b = b0 + lane;
+    const unsigned x = b < nblocks ? row[b] : 0u;
+    unsigned incl = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (b < nblocks) row[b] = carry + incl - x;
+    carry += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (lane == 0) totals[d] = carry;
+}
+
+// Stable scatter of a tile: a warp owns 32 kSortItems keys in a row.
+__global__ void __launch_bounds__(kSortThreads)
+topk_sort_scatter_kernel(const unsigned int* in, unsigned int* out, unsigned long long k,
+                         const TopkState* st, int pass, const unsigned int* hist, int nblocks,
+                         const unsigned int* totals) {
+  constexpr int kWarps = kSortThreads / 32;
+  __shared__ unsigned int s_w[kWarps][256];  // per warp: count, then first slot
+  __shared__ unsigned int s_sum[kWarps];
+  if (pass >= topk_passes(st)) return;
+  const unsigned kk = topk_k(st, k);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (int w = 0; w < kWarps; ++w) s_w[w][threadIdx.x] = 0;
+  // first slot of digit threadIdx.x: the totals of the digits below it
+  const unsigned tot = totals[threadIdx.x];
+  unsigned incl = tot;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_sum[wid] = incl;
+  __syncthreads();
+  unsigned first = incl - tot;
+  for (int w = 0; w < wid; ++w) first += s_sum[w];
+  const unsigned long long base =
+      static_cast<unsigned long long>(blockIdx.x) * kSortTile + wid * (32 * kSortItems);
+  unsigned key[kSortItems], rank[kSortItems];
+#pragma unroll
+  for (int t = 0; t < kSortItems; ++t) {
+    const unsigned long long i = base + t * 32 + lane;
+    const bool on = i < kk;
+    key[t] = on ? in[i] : 0u;
+    const unsigned d = on ? (key[t] >> (8 * pass)) & 255u : 256u;
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    // the warp's earlier keys of this digit, then its earlier lanes
+    const unsigned before = on ? s_w[wid][d] : 0u;
+    rank[t] = before + __popc(peers & lanemask_lt());
+    __syncwarp();
+    if (on && lane == __ffs(peers) - 1) s_w[wid][d] = before + __popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  unsigned at = first + hist[static_cast<size_t>(threadIdx.x) * nblocks + blockIdx.x];
+  for (int w = 0; w < kWarps; ++w) {
+    const unsigned c = s_w[w][threadIdx.x];
+    s_w[w][threadIdx.x] = at;
+    at += c;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < kSortItems; ++t) {
+    const unsigned long long i = base + t * 32 + lane;
+    if (i < kk) out[s_w[wid][(key[t] >> (8 * pass)) & 255u] + rank[t]] = key[t];
+  }
+}
+
+__global__ void topk_emit_kernel(const unsigned int* a, const unsigned int* b,
+                                 unsigned long long k, const TopkState* st, float* out) {
+  const unsigned kk = topk_k(st, k);
+  const unsigned lo = ~__ldcg(&st->inv_min);
+  const unsigned int* keys = topk_passes(st) & 1 ? b : a;
   for (unsigned long long i = static_cast<unsigned long long>(blockIdx.x) * blockDim.x +
                               threadIdx.x;
-       i < n; i += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
-    out[i] = key_float(keys[i]);
+       i < kk; i += static_cast<unsigned long long>(gridDim.x) * blockDim.x)
+    out[i] = key_float(keys[i] + lo);
 }
 
 }  // namespace
 
 size_t topk_sort_hist_words(unsigned long long k) {
-  return 256 * ((k + kSortTile - 1) / kSortTile);
+  return 256 * ((k + kSortTile - 1) / kSortTile) + 256;
 }
 
-// The k smallest non-zero values of costs[0..n), ascending, into out.  Two
-// stages separated by a host read of the non-zero count: count, then select
-// + compact + sort + gather.  s.hist must hold 2048 zero words (the select
-// leaves them zero again); s.keys/s.vals 2*k words each.
+// The k smallest non-zero values of costs[0..n), ascending, into out; waits
+// for the stream to learn how many there are.  s.hist must hold kTopkBins zero
+// words (the select leaves them zero again); s.keys 2*k words.
 int launch_topk_costs(const float* costs, unsigned long long n, unsigned long long k,
                       const TopkScratch& s, float* out, unsigned long long* n_out,
                       void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   *n_out = 0;
   if (n == 0 || k == 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(s.counts, 0, 2 * sizeof(unsigned long long), st);
+  TopkState* ts = static_cast<TopkState*>(s.state);
+  cudaError_t e = cudaMemsetAsync(ts, 0, sizeof(TopkState), st);
   if (e != cudaSuccess) return e;
-  const unsigned int all = 0xffffffffu;
-  e = cudaMemcpyAsync(s.tkey, &all, 4, cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return e;
-  count_le_kernel<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(costs, n, 1, s.tkey, s.counts);
-  unsigned long long host_counts[2] = {0, 0};
-  e = cudaMemcpyAsync(host_counts, s.counts, sizeof(host_counts), cudaMemcpyDeviceToHost, st);
-  if (e != cudaSuccess) return e;
-  e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) return e;
-  const unsigned long long kk = host_counts[1] < k ? host_counts[1] : k;
-  *n_out = kk;
-  if (kk == 0) return cudaSuccess;
-  int launches = 0;
-  e = static_cast<cudaError_t>(launch_select_kth(costs, n, 1, nullptr, 0, 1, kk, 1, s.state,
-                                                 s.hist, st, &launches));
-  if (e != cudaSuccess) return e;
-  cudaMemsetAsync(s.cnt, 0, 2 * sizeof(unsigned long long), st);
-  cudaMemsetAsync(s.vals, 0, kk * sizeof(unsigned int), st);
-  compact_kernel<<<grid_for(n, 256, 148 * 16), 256, 0, st>>>(
-      costs, n, static_cast<const SelectState*>(s.state), kk, s.keys, s.vals, s.cnt);
-  const int nblocks = static_cast<int>((kk + kSortTile - 1) / kSortTile);
-  unsigned int* kin = s.keys;
-  unsigned int* vin = s.vals;
-  unsigned int* kout = s.keys + kk;
-  unsigned int* vout = s.vals + kk;
+  const int grid = grid_for(n, kTopkThreads * 8, 148 * 2);
+  topk_range_kernel<<<grid, kTopkThreads, 0, st>>>(costs, n, ts);
+  for (int digit = 0; digit < 3; ++digit)
+    topk_digit_kernel<<<grid, kTopkThreads, 0, st>>>(costs, n, k, ts, s.hist, digit == 0);
+  topk_compact_kernel<<<grid, kTopkThreads, 0, st>>>(costs, n, k, ts, s.keys);
+  const int nblocks = static_cast<int>((k + kSortTile - 1) / kSortTile);
+  unsigned int* totals = s.sort_hist + static_cast<size_t>(256) * nblocks;
   for (int pass = 0; pass < 4; ++pass) {
-    const int shift = pass * 8;
-    sort_hist_kernel<<<nblocks, kSortThreads, 0, st>>>(kin, kk, shift, s.sort_hist, nblocks);
-    sort_scan_kernel<<<1, 1024, 0, st>>>(s.sort_hist, 256 * nblocks);
-    sort_scatter_kernel<<<nblocks, kSortThreads, 0, st>>>(kin, vin, kout, vout, kk, shift,
-                                                          s.sort_hist, nblocks);
-    unsigned int* t = kin;
-    kin = kout;
-    kout = t;
-    t = vin;
-    vin = vout;
-    vout = t;
+    const unsigned int* in = s.keys + (pass & 1 ? k : 0);
+    unsigned int* to = s.keys + (pass & 1 ? 0 : k);
+    topk_sort_hist_kernel<<<nblocks, kSortThreads, 0, st>>>(in, k, ts, pass, s.sort_hist, nblocks);
+    topk_sort_rows_kernel<<<32, 256, 0, st>>>(ts, pass, s.sort_hist, nblocks, totals);
+    topk_sort_scatter_kernel<<<nblocks, kSortThreads, 0, st>>>(in, to, k, ts, pass, s.sort_hist,
+                                                               nblocks, totals);
   }
-  keys_to_costs_kernel<<<grid_for(kk, 256, 148 * 8), 256, 0, st>>>(kin, kk, out);
-  return cudaGetLastError();
+  topk_emit_kernel<<<grid_for(k, 256, 148 * 8), 256, 0, st>>>(s.keys, s.keys + k, k, ts, out);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  unsigned int nz = 0;
+  e = cudaMemcpyAsync(&nz, &ts->nz, sizeof(nz), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) *n_out = k < nz ? k : nz;
+  return e;
 }
 
 }  // namespace cpg
@@ -447,7 +773,7 @@ int launch_topk_costs(const float* costs, unsigned long long n, unsigned long lo
 // ---------------------------------------------------------------- no-alloc
 // cpg_select_topk_noalloc: the same top-K as cpg_select_topk, for callers
 // that must not allocate device memory.  Its scratch is this file-scope
-// array, reserved when the library is loaded (4.3 MiB on every GPU that
+// array, reserved when the library is loaded (2.2 MiB on every GPU that
 // loads it, held until the process exits).  In host code the name
 // g_topk_scratch is only a host-side stand-in: the kernels get the device
 // address that cudaGetSymbolAddress returns, looked up once per device with
@@ -456,10 +782,10 @@ namespace cpg {
 namespace {
 
 constexpr unsigned long long kNoAllocMaxK = CPG_SELECT_TOPK_NOALLOC_MAX_K;
-// hist 2048 + state 4 + counts 4 + cnt 4 + tkey 4, keys/vals 2*K each,
-// sort histogram 256 * ceil(K / 2048)
+// hist 2048, state, keys 2*K, sort histogram 256 * (ceil(K / 2048) + 1)
 constexpr size_t kNoAllocWords =
-    2048 + 16 + 4 * kNoAllocMaxK + 256 * ((kNoAllocMaxK + kSortTile - 1) / kSortTile);
+    2048 + kTopkStateWords + 2 * kNoAllocMaxK +
+    256 * ((kNoAllocMaxK + kSortTile - 1) / kSortTile + 1);
 
 __device__ __align__(256) unsigned int g_topk_scratch[kNoAllocWords];
 
@@ -505,12 +831,8 @@ extern "C" cpg_status cpg_select_topk_noalloc(const float* d_costs, int64_t n,
   TopkScratch sc;
   sc.hist = w;
   sc.state = w + 2048;
-  sc.counts = reinterpret_cast<unsigned long long*>(w + 2048 + 4);
-  sc.cnt = reinterpret_cast<unsigned long long*>(w + 2048 + 8);
-  sc.tkey = w + 2048 + 12;
-  sc.keys = w + 2048 + 16;
-  sc.vals = sc.keys + 2 * kNoAllocMaxK;
-  sc.sort_hist = sc.vals + 2 * kNoAllocMaxK;
+  sc.keys = w + 2048 + kTopkStateWords;
+  sc.sort_hist = sc.keys + 2 * kNoAllocMaxK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // the array keeps the previous call's contents: the select histogram must
   // start at zero

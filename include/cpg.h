@@ -391,7 +391,8 @@ cpg_status cpg_server_get_stats(const cpg_server* s, cpg_server_stats* out);
  * nodes (gpucpg.cu:21323-21360); here a radix select finds the k-th value and
  * only the k survivors are radix-sorted.  Runs on `stream` (a cudaStream_t,
  * NULL for the default stream) and returns after the result is written.
- * Allocates and frees its own device scratch. */
+ * Its device scratch comes from a stream-ordered pool of the library's own,
+ * one per device, which keeps at most 32 MiB between calls. */
 cpg_status cpg_select_topk(const float* d_costs, int64_t n, int64_t k,
                            float* d_out, int64_t* n_out, void* stream);
 
@@ -400,7 +401,7 @@ cpg_status cpg_select_topk(const float* d_costs, int64_t n, int64_t k,
 
 /* cpg_select_topk for callers that cannot allocate device memory: the same
  * k smallest non-zero costs, ascending, but its scratch is a fixed array
- * inside the library instead of cudaMalloc/cudaFree.  Meant for code that
+ * inside the library instead of pool memory.  Meant for code that
  * runs where an allocation is not allowed or not affordable: between the
  * kernels of a pipeline whose other streams must keep running (cudaFree
  * synchronises the whole device), under a memory pool or budget that owns
@@ -411,7 +412,7 @@ cpg_status cpg_select_topk(const float* d_costs, int64_t n, int64_t k,
  * Limits and rules:
  *  - k <= CPG_SELECT_TOPK_NOALLOC_MAX_K, else CPG_ERR_CAPACITY (nothing runs);
  *    n < 2^32.
- *  - The scratch (about 4.3 MiB) is reserved on every GPU that loads the
+ *  - The scratch (about 2.2 MiB) is reserved on every GPU that loads the
  *    library and kept until the process exits.
  *  - No call can run inside a stream capture: every call reads the count of
  *    non-zero costs back to the host partway through and synchronises

@@ -36,3 +36,27 @@ def test_select_topk_all_zero_and_empty():
     out = torch.empty(10, dtype=torch.float32, device="cuda")
     assert cpg_b200.select_topk(d.data_ptr(), 1000, 10, out.data_ptr()) == 0
     assert cpg_b200.select_topk(d.data_ptr(), 0, 10, out.data_ptr()) == 0
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("values", ["one", "two_bits", "few", "narrow", "signs", "inf", "all_bits"])
+@pytest.mark.parametrize("n,k", [(1, 3), (5, 2), (2047, 2048), (8193, 2049), (300_001, 70_000)])
+def test_select_topk_over_key_ranges_and_alignments(n, k, values, offset):
+    """Inputs whose keys differ in no bit, few bits or all 32, values of both
+    signs and infinities, at every offset from a 16-byte boundary."""
+    import torch
+    rng = np.random.default_rng(n + offset)
+    c = {"one": lambda: np.full(n, 7.25),
+         "two_bits": lambda: rng.choice([1.0, 1.0000001, 1.0000002], n),
+         "few": lambda: rng.integers(1, 5, n),
+         "narrow": lambda: rng.uniform(40.0, 40.01, n),
+         "signs": lambda: rng.normal(0.0, 3.0, n),
+         "inf": lambda: rng.choice([-np.inf, np.inf, 1.0, 0.0, -0.0, 3e38], n),
+         "all_bits": lambda: rng.choice([-3e38, -1e-40, 1e-40, 2.0, 3e38], n)}[values]().astype(np.float32)
+    d = torch.zeros(n + offset, dtype=torch.float32, device="cuda")
+    d[offset:] = torch.from_numpy(c).cuda()
+    out = torch.full((k,), -1.0, dtype=torch.float32, device="cuda")
+    got = cpg_b200.select_topk(d.data_ptr() + 4 * offset, n, k, out.data_ptr())
+    want = np.sort(c[c != 0.0])[:k]
+    assert got == want.size
+    assert np.array_equal(out[:got].cpu().numpy().view(np.uint32), want.view(np.uint32))
