@@ -397,7 +397,8 @@ struct EngineQuery {
   unsigned long long k_out, out_off, out_lt, out_eq;
   int phases;
   int whole;                  // answered by its own block (engine_block_kernel)
-  unsigned long long acc_prev, last_j;  // accepted before / promoted in the last growth phase
+  // the last growth phase: accepted before it, promoted, of how many pending
+  unsigned long long acc_prev, last_j, last_pend;
   // set by the host: where the query's costs go, and its block's share of the
   // path store and of the global overflow of its piles
   unsigned long long path_base, path_cap, pend_base, pend_cap, front_base, front_cap;
@@ -456,7 +457,7 @@ struct EngineParams {
   EngineCounters* ctr;
   unsigned int spin_limit;
   int grid_limit;             // persistent CTAs (0: one per co-resident slot)
-  int grow_cap_k;             // cap a growth phase's promotion at K - accepted
+  int grow_cap_k;             // a growth phase near K aims at K
   // a block leaves a query that is not `whole` to the grid launch once more
   // items than this are pending
   unsigned long long solo_stop;
