@@ -47,15 +47,23 @@ struct alignas(8) DevEdge {
 };
 
 // One deviation ("sidetrack") edge (v, head) with head != succ[v]: the delay,
-// the head's fixed-point distance and the sort key (its cost increase).  Each
-// vertex's deviations are stored ascending by key in its own fan-out slots, so
-// the list is also a binary min-heap (children 2j+1, 2j+2).
+// the head's fixed-point distance and, while rows are built and sorted, the
+// key (its cost increase).
+//
+// A stored row is a heap over v's own fan-out slots.  Its first H entries are
+// ascending, so they are a binary min-heap (children 2j+1, 2j+2 below H);
+// behind them come side lists, each ascending and no cheaper than the heap
+// entry it hangs from.  In a stored row `key` holds the index of an entry's
+// side child as an int, or -1.  dev_cnt[v] is H, with kDevSide set when entry
+// 0 has a side list, which then starts at index H.  Rows of up to 32
+// deviations, sorted rows and rows of more than 256 edges have no side lists.
 struct alignas(16) DevSidetrack {
   int32_t head;
   float w;
   int32_t dist_head;
   float key;
 };
+constexpr int kDevSide = 1 << 30;
 
 // Node of the persistent chain heap: the heap of vertex v holds, for every
 // vertex u on v's suffix chain that has deviations, u's cheapest deviation.

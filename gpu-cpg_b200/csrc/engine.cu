@@ -598,13 +598,14 @@ __device__ __forceinline__ unsigned long long warp_reserve(unsigned long long* c
   return base + (incl - n);
 }
 
-// An accepted item as a path, and its (up to) five children: heap left /
-// right (or row 2j+1 / 2j+2), row entries 1 and 2 of a heap node's row, and
-// the cross child.
+// An accepted item as a path, and its (up to) six children: heap left /
+// right (or row 2j+1 / 2j+2), row entries 1 and 2 of a heap node's row, the
+// cross child, and the row entry's side child.
+constexpr int kKids = 6;
 struct Grown {
   HeapNode hn;
-  int cross;
-  float cc[5];
+  int cross, side;
+  float cc[kKids];
   unsigned tm, dm;  // children at or below the limit, and above it
   bool stored;
 };
@@ -630,12 +631,13 @@ __device__ __forceinline__ Grown grow_path(const EngineParams& p, const Item& it
   const bool dev = g.stored && it.node >= 0;
   int to = -1, from = -1, level = 0;
   float pcost = 0.f;
+  g.side = -1;
   if (dev) {
     g.hn = load_node(p.g.hnodes, it.node);
     level = __ldcg(p.ps.level + it.parent) + 1;
     pcost = __ldcg(p.ps.cost + it.parent);
     from = g.hn.vtx;
-    to = dev_head(p.g, g.hn, jj);
+    to = dev_head(p.g, g.hn, jj, g.side);
   } else if (g.stored) {
     to = -(it.node + 2);
   }
@@ -653,9 +655,10 @@ __device__ __forceinline__ Grown grow_path(const EngineParams& p, const Item& it
   if (sib && jj == 0 && cand_row(p.g, g.hn, 1, pcost, g.cc[2])) exm |= 4u;
   if (sib && jj == 0 && cand_row(p.g, g.hn, 2, pcost, g.cc[3])) exm |= 8u;
   if (expand && cand_top(p.g, g.cross, it.cost, g.cc[4])) exm |= 16u;
+  if (sib && cand_side(p.g, g.hn, g.side, pcost, g.cc[5])) exm |= 32u;
   g.tm = g.dm = 0;
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
+  for (int k = 0; k < kKids; ++k) {
     if (!(exm & (1u << k))) continue;
     if (g.cc[k] <= lim) g.tm |= 1u << k;
     else g.dm |= 1u << k;
@@ -679,7 +682,8 @@ __device__ __forceinline__ Item child_of(const Grown& g, const Item& it, unsigne
   c.cost = g.cc[k];
   c.parent = k == 4 ? static_cast<int>(qp) : it.parent;
   c.node = k == 4 ? g.cross : (k < 2 && jj == 0 ? (k == 0 ? g.hn.left : g.hn.right) : it.node);
-  c.j = pack_j(q, k == 4 ? 0 : k == 2 ? 1 : k == 3 ? 2 : (jj == 0 ? 0 : 2 * jj + 1 + k));
+  c.j = pack_j(q, k == 5 ? g.side : k == 4 ? 0 : k == 2 ? 1 : k == 3 ? 2
+                  : jj == 0 ? 0 : 2 * jj + 1 + k);
   return c;
 }
 
@@ -687,7 +691,7 @@ __device__ __forceinline__ Item child_of(const Grown& g, const Item& it, unsigne
 __device__ __forceinline__ unsigned pending_nz(const Grown& g) {
   unsigned n = 0;
 #pragma unroll
-  for (int k = 0; k < 5; ++k) n += ((g.dm >> k) & 1u) && g.cc[k] != 0.0f;
+  for (int k = 0; k < kKids; ++k) n += ((g.dm >> k) & 1u) && g.cc[k] != 0.0f;
   return n;
 }
 
@@ -729,11 +733,11 @@ __device__ bool run_closure(const EngineParams& p, Item* pend_out) {
                                 single || !valid ? tie0 : __ldcg(&p.q[q].tie));
       if (single) acc_nz += g.stored && it.cost != 0.0f;
       else qadd(p.q, QOFF(paths_nz), g.stored && it.cost != 0.0f, q, 1u);
-      // one reservation per warp and counter for all five
+      // one reservation per warp and counter for all of them
       unsigned long long bt = warp_reserve(out_cnt, __popc(g.tm));
       unsigned long long bd = warp_reserve(&p.ctr->pend_out, __popc(g.dm));
 #pragma unroll
-      for (int k = 0; k < 5; ++k) {
+      for (int k = 0; k < kKids; ++k) {
         const unsigned bit = 1u << k;
         if (!((g.tm | g.dm) & bit)) continue;
         const Item c = child_of(g, it, q, qp, k);
@@ -1497,7 +1501,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
         unsigned bt = blk_reserve(&s_front[(r + 1) % 3], __popc(g.tm));
         unsigned bd = blk_reserve(&s_pend[pin ^ 1], __popc(g.dm));
 #pragma unroll
-        for (int k = 0; k < 5; ++k) {
+        for (int k = 0; k < kKids; ++k) {
           const unsigned bit = 1u << k;
           if (!((g.tm | g.dm) & bit)) continue;
           const Item c = child_of(g, it, q, qp, k);

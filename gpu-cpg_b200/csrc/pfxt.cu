@@ -82,7 +82,7 @@ closure_kernel(ClosureParams p) {
       // accept: materialise the path
       const unsigned long long q = warp_append(&p.ctr->paths, valid);
       bool stored = false;
-      int to = -1;
+      int to = -1, link = -1;
       HeapNode hn;
       hn.vtx = -1;
       hn.left = -1;
@@ -99,7 +99,7 @@ closure_kernel(ClosureParams p) {
         } else {
           hn = load_node(p.g.hnodes, it.node);
           from = hn.vtx;
-          to = dev_head(p.g, hn, it.j);
+          to = dev_head(p.g, hn, it.j, link);
           level = __ldcg(p.ps.level + it.parent) + 1;
         }
         if (q < p.ps.cap) {
@@ -141,6 +141,10 @@ closure_kernel(ClosureParams p) {
         route(p, out, out_cnt, ex, c);
         c.j = 2;
         ex = sib && it.j == 0 && cand_row(p.g, hn, c.j, pcost, c.cost);
+        route(p, out, out_cnt, ex, c);
+        // the entry's side list
+        c.j = link;
+        ex = sib && cand_side(p.g, hn, link, pcost, c.cost);
         route(p, out, out_cnt, ex, c);
       }
       // cross: the cheapest deviation on the new path's own suffix chain

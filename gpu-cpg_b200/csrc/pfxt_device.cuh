@@ -65,23 +65,40 @@ __device__ __forceinline__ bool cand_top(const PfxtGraph& g, int node, float par
   return true;
 }
 
-// Candidate (entry j >= 1 of the sorted row of hn's vertex).  The entry and
-// the row's count are requested together (rows are padded, so the entry's
-// load stays inside the allocation for any j a search asks); false if j is
-// past the count.
+// Candidate (entry j >= 1 of the heap part of the row of hn's vertex).  The
+// entry and the row's count are requested together (rows are padded, so the
+// entry's load stays inside the allocation for any j a search asks); false if
+// j is past the heap part.
 __device__ __forceinline__ bool cand_row(const PfxtGraph& g, const HeapNode& hn, int j,
                                          float parent_cost, float& cost) {
-  const int cnt = __ldg(g.dev_cnt + hn.vtx);
+  const int cnt = __ldg(g.dev_cnt + hn.vtx) & (kDevSide - 1);
   const DevSidetrack d = load_dev(g.dev, hn.row + j);
   if (j >= cnt) return false;
   cost = child_cost(g.division, parent_cost, d.dist_head, d.w, hn.dist_v);
   return true;
 }
 
-// Head of entry j of the sorted row of hn's vertex: the last edge of the
-// path that takes that deviation.
-__device__ __forceinline__ int dev_head(const PfxtGraph& g, const HeapNode& hn, int j) {
-  return j == 0 ? hn.head : load_dev(g.dev, hn.row + j).head;
+// Candidate (entry `link` of the row, an entry's side child); false if -1.
+__device__ __forceinline__ bool cand_side(const PfxtGraph& g, const HeapNode& hn, int link,
+                                          float parent_cost, float& cost) {
+  if (link < 0) return false;
+  const DevSidetrack d = load_dev(g.dev, hn.row + link);
+  cost = child_cost(g.division, parent_cost, d.dist_head, d.w, hn.dist_v);
+  return true;
+}
+
+// Entry j of the row of hn's vertex: the head (the last edge of the path that
+// takes that deviation), and the index of its side child or -1.
+__device__ __forceinline__ int dev_head(const PfxtGraph& g, const HeapNode& hn, int j,
+                                        int& link) {
+  if (j == 0) {
+    const int cnt = __ldg(g.dev_cnt + hn.vtx);
+    link = cnt & kDevSide ? cnt & (kDevSide - 1) : -1;
+    return hn.head;
+  }
+  const DevSidetrack d = load_dev(g.dev, hn.row + j);
+  link = __float_as_int(d.key);
+  return d.head;
 }
 
 }  // namespace cpg

@@ -151,6 +151,12 @@ __device__ __forceinline__ void warp_sort_regs(unsigned long long (&x)[C]) {
   }
 }
 
+// An entry of a stored row without a side list.
+__device__ __forceinline__ void store_entry(DevSidetrack* at, DevSidetrack r) {
+  r.key = __int_as_float(-1);
+  *at = r;
+}
+
 // A row the build left unsorted, for sort_rows_kernel.
 __device__ __forceinline__ void list_long_row(const SfxtParams& p, int v) {
   p.long_rows[atomicAdd(&p.ctr->n_long, 1)] = v;
@@ -176,7 +182,7 @@ __device__ __forceinline__ void sort_row_words(DevSidetrack* row, int cnt) {
   __syncwarp();
 #pragma unroll
   for (int c = 0; c < C; ++c)
-    if (c * 32 + lane < cnt) row[c * 32 + lane] = o[c];
+    if (c * 32 + lane < cnt) store_entry(&row[c * 32 + lane], o[c]);
   __syncwarp();
 }
 
@@ -200,7 +206,7 @@ __device__ __forceinline__ void sort_row_regs(DevSidetrack* row, int cnt) {
     o.w = __shfl_sync(0xffffffffu, r.w, src & 31);
     o.dist_head = __shfl_sync(0xffffffffu, r.dist_head, src & 31);
     o.key = __shfl_sync(0xffffffffu, r.key, src & 31);
-    if (lane < cnt) row[lane] = o;
+    if (lane < cnt) store_entry(&row[lane], o);
     return;
   }
   sort_row_words<4>(row, cnt);
@@ -222,7 +228,7 @@ __device__ __forceinline__ int write_short_row(const SfxtParams& p, int rb, bool
   o.dist_head = __shfl_sync(0xffffffffu, rec.dist_head, src);
   o.key = __shfl_sync(0xffffffffu, rec.key, src);
   const int cnt = __popc(bal);
-  if (lane < cnt) p.dev[rb + lane] = o;
+  if (lane < cnt) store_entry(p.dev + rb + lane, o);
   top = o;
   return cnt;
 }
@@ -276,7 +282,7 @@ __device__ __forceinline__ int write_row64(const SfxtParams& p, int rb, bool v0,
     o.dist_head = hi ? d1 : d0;
     o.key = hi ? k1 : k0;
     const int i = 32 * c + lane;
-    if (i < cnt) p.dev[rb + i] = o;
+    if (i < cnt) store_entry(p.dev + rb + i, o);
     if (c == 0) top = o;
   }
   return cnt;
@@ -476,7 +482,7 @@ __device__ int build_vertex(const SfxtParams& p, int v, int lvl, bool do_kahn) {
     p.dist[v] = best;
     p.succ[v] = s;
     p.dev_cnt[v] = cnt;
-    if (re - rb > 64 && cnt > 1 && cnt <= kSmemRow) list_long_row(p, v);
+    if (re - rb > 64 && cnt > 0 && cnt <= kSmemRow) list_long_row(p, v);
     // the chain-heap insert, one level later, takes v's cheapest deviation
     if (cnt > 0) p.best[v] = top;
     if (kLevel) p.level_of[v] = lvl;
@@ -611,7 +617,7 @@ __device__ void build_group(const SfxtParams& p, int v, int lvl, bool do_kahn) {
   o.w = __shfl_sync(0xffffffffu, rec.w, src);
   o.dist_head = __shfl_sync(0xffffffffu, rec.dist_head, src);
   o.key = __shfl_sync(0xffffffffu, rec.key, src);
-  if (has_v && l < cnt) p.dev[rb + l] = o;
+  if (has_v && l < cnt) store_entry(p.dev + rb + l, o);
   if (has_v && l == 0) {
     p.dist[v] = best;
     p.succ[v] = s;
@@ -1160,6 +1166,96 @@ __device__ __forceinline__ void publish_dl(const SfxtParams& p, int v, int lvl, 
         static_cast<unsigned>(best);
 }
 
+// Stores a row of 33 to 32 C edges held C to a lane: every lane's cheapest
+// deviation goes to the heap part, sorted across the lanes by one 32-word
+// network whatever C is, and a lane's others to its side list, ordered by
+// counting (no shuffles).  A whole sort took a pass of its own over rows of
+// more than 64 edges, which read them back and wrote them again (suffix tree
+// with that pass 2.95 -> 2.25 ms at mean degree 50, 1.69 -> 1.58 at 20, both 1M
+// pins; a search finds one child more per item that has a side list).
+// Returns dev_cnt; every lane's top is the row's cheapest deviation.
+template <int C>
+__device__ __forceinline__ int write_side_row(const SfxtParams& p, int rb, const DevEdge (&ed)[C],
+                                              const int (&dh)[C], int succ, int best,
+                                              DevSidetrack& top) {
+  const int lane = threadIdx.x & 31;
+  unsigned key[C];  // orderable keys; a slot without a deviation is none
+  int mine = 0;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const bool valid = ed[c].head >= 0 && ed[c].head != succ && dh[c] != INT_MAX;
+    // (a delay of NaN has the largest key there is: still before none)
+    key[c] = valid ? min(float_key(deviation_key(dh[c], best, ed[c].w)), 0xfffffffeu)
+                   : 0xffffffffu;
+    mine += valid;
+  }
+  // each slot's rank in its lane (edge order among equal keys; an empty slot
+  // ranks behind every deviation)
+  int rank[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    rank[c] = 0;
+#pragma unroll
+    for (int d = 0; d < C; ++d)
+      if (d != c) rank[c] += key[d] < key[c] || (key[d] == key[c] && d < c);
+  }
+  DevSidetrack first;  // this lane's cheapest
+  first.head = -1;
+  first.w = 0.f;
+  first.dist_head = 0;
+  unsigned fk = 0xffffffffu, fc = 0;
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (rank[c] == 0) {
+      first.head = ed[c].head;
+      first.w = ed[c].w;
+      first.dist_head = dh[c];
+      fk = key[c];
+      fc = c;
+    }
+  const unsigned some = __ballot_sync(0xffffffffu, mine > 0);
+  const int H = __popc(some);
+  // heads in order: lane i < H learns the lane whose head is i-th ...
+  const unsigned long long x =
+      warp_sort32(mine > 0 ? (static_cast<unsigned long long>(fk) << 32) | (fc * 32 + lane) : ~0ull);
+  const int from = static_cast<int>(x & 31u);
+  // ... and every lane its own head's place
+  unsigned at = H == 32 ? 0xffffffffu : (1u << H) - 1u;
+#pragma unroll
+  for (int b = 0; b < 5; ++b) {
+    const unsigned m = __ballot_sync(0xffffffffu, (from >> b) & 1);
+    at &= (lane >> b) & 1 ? m : ~m;
+  }
+  const int place = __ffs(at) - 1;
+  // side lists: the first head's at H, the others' behind it, lane by lane
+  const int side = mine > 1 ? mine - 1 : 0;
+  const int side0 = __shfl_sync(0xffffffffu, side, H ? __shfl_sync(0xffffffffu, from, 0) : 0);
+  int incl = place == 0 ? 0 : side;
+  const int own = incl;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  const int base = place == 0 ? H : H + side0 + incl - own;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    if (rank[c] >= mine) continue;
+    DevSidetrack r;
+    r.head = ed[c].head;
+    r.w = ed[c].w;
+    r.dist_head = dh[c];
+    r.key = __int_as_float(rank[c] + 1 < mine ? base + rank[c] : -1);
+    p.dev[rb + (rank[c] == 0 ? place : base + rank[c] - 1)] = r;
+  }
+  const int f0 = __shfl_sync(0xffffffffu, from, 0);
+  top.head = __shfl_sync(0xffffffffu, first.head, f0);
+  top.w = __shfl_sync(0xffffffffu, first.w, f0);
+  top.dist_head = __shfl_sync(0xffffffffu, first.dist_head, f0);
+  top.key = deviation_key(top.dist_head, best, top.w);
+  return H | (H > 0 && side0 > 0 ? kDevSide : 0);
+}
+
 // Early-push build of a row of at most 32 C edges: the whole row in registers,
 // C words a lane.  best, s, cnt, lmax and top are build_vertex_polled's; false
 // if a wait ran out (warp-uniform).  One copy per C: a warp issues a dependent
@@ -1261,37 +1357,8 @@ __device__ __forceinline__ bool build_row_polled(const SfxtParams& p, int v, int
     rec.dist_head = dh[0];
     rec.key = deviation_key(dh[0], best, ed[0].w);
     cnt = write_short_row(p, rb, valid, rec, top);
-  } else if constexpr (C == 2) {
-    DevSidetrack r[2];
-    bool v[2];
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      v[c] = ed[c].head >= 0 && ed[c].head != s && dh[c] != INT_MAX;
-      r[c].head = ed[c].head;
-      r[c].w = ed[c].w;
-      r[c].dist_head = dh[c];
-      r[c].key = deviation_key(dh[c], best, ed[c].w);
-    }
-    cnt = write_row64(p, rb, v[0], r[0], v[1], r[1], top);
   } else {
-    BestDev bd = best_none();
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      if (rb + c * 32 >= re) break;
-      const bool valid = ed[c].head >= 0 && ed[c].head != s && dh[c] != INT_MAX;
-      const unsigned bal = __ballot_sync(0xffffffffu, valid);
-      if (valid) {
-        DevSidetrack rec;
-        rec.head = ed[c].head;
-        rec.w = ed[c].w;
-        rec.dist_head = dh[c];
-        rec.key = deviation_key(dh[c], best, ed[c].w);
-        p.dev[rb + cnt + __popc(bal & lanemask_lt())] = rec;
-        best_take(bd, true, rec, c * 32 + lane);
-      }
-      cnt += __popc(bal);
-    }
-    top = best_reduce(bd);
+    cnt = write_side_row<C>(p, rb, ed, dh, s, best, top);
   }
   lmax = lvl;
   return true;
@@ -1413,7 +1480,7 @@ __device__ int build_vertex_polled(const SfxtParams& p, int v, int rb, int re, D
     p.dist[v] = best;
     p.succ[v] = s;
     p.dev_cnt[v] = cnt;
-    if (re - rb > 64 && cnt > 1 && cnt <= kSmemRow) list_long_row(p, v);
+    if (re - rb > kRegChunks * 32 && cnt > 0 && cnt <= kSmemRow) list_long_row(p, v);
     if (cnt > 0) p.best[v] = top;
     p.level_of[v] = lmax;
   }
@@ -2004,7 +2071,7 @@ sort_rows_kernel(const int32_t* rows, const int* n_rows, const int32_t* adjp,
       }
     }
     for (int t = lane; t < cnt; t += 32)
-      row[t] = srec[w][static_cast<int>(skey[w][t] & 0xffffffffu)];
+      store_entry(&row[t], srec[w][static_cast<int>(skey[w][t] & 0xffffffffu)]);
     __syncwarp();
   }
 }
@@ -2054,7 +2121,7 @@ __global__ void sort_big_rows_kernel(const int32_t* rows, const int32_t* adjp,
     }
   }
   for (int t = threadIdx.x; t < cnt; t += blockDim.x)
-    row[t] = tmp[static_cast<int>(wbuf[t] & 0xffffffffu)];
+    store_entry(&row[t], tmp[static_cast<int>(wbuf[t] & 0xffffffffu)]);
 }
 
 }  // namespace
