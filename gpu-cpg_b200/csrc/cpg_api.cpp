@@ -2566,6 +2566,26 @@ cpg_status cpg_server_start(cpg_server* sv) {
   if (!sv || sv->running) return CPG_ERR_INVALID;
   cpg_status st = cpg_batch_commit(sv->b);
   if (st != CPG_OK) return st;
+  {
+    // Rebuilds after delay updates append their chain heaps to the pool, and
+    // one that overflows it is done again for every graph: room for two more
+    // trees (a tree takes about 7 nodes a vertex, the pool has 10), if the
+    // device has it to spare.
+    cpg_handle* h = sv->b->h;
+    const unsigned long long want = h->hnode_cap + 14ull * static_cast<unsigned long long>(h->g.n);
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want * sizeof(HeapNode) < free_b / 4) {
+      const unsigned long long had = h->hnode_cap;
+      release(h->d_hnodes);
+      h->hnode_cap = want;
+      if (ensure(h->d_hnodes, want * sizeof(HeapNode)) != cudaSuccess) {
+        cudaGetLastError();
+        h->hnode_cap = had;
+        const Status ws = ensure(h->d_hnodes, had * sizeof(HeapNode)) == cudaSuccess ? CPG_OK : CPG_ERR_OOM;
+        if (ws != CPG_OK) return fail(h, ws, "alloc chain heaps");
+      }
+    }
+  }
   st = cpg_levelize(sv->b->h);
   if (st != CPG_OK) return st;
   // The engine's path and item piles, sized once for a launch answering
