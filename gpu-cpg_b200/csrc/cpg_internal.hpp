@@ -205,7 +205,7 @@ struct SfxtParams {
   // full CSR builds: dataflow work queue unless level_sync is set
   int32_t* queue;          // 32 << queue_shift ints >= n
   int32_t queue_shift;
-  int32_t* long_rows;      // rows over 64 edges, written unsorted (n ints)
+  int32_t* long_rows;      // rows written unsorted, for sort_rows_kernel (n ints)
   int32_t level_sync;
   int32_t heap_warps;      // dataflow: warps per CTA that only insert heaps (0: none)
   int32_t early_push;      // dataflow: push tails before the build, poll dl[]

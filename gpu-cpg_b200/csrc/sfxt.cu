@@ -213,8 +213,8 @@ __device__ __forceinline__ void sort_row_regs(DevSidetrack* row, int cnt) {
 }
 
 // A row of at most 32 edges (one per lane) is sorted in registers and
-// written once, in order (write_row64 does the same up to 64 edges); longer
-// rows are written in edge order and sorted by sort_rows_kernel.  Returns the
+// written once, in order (write_row64 does the same up to 64 edges in the
+// level-synchronous build, write_side_row from 33 edges on in the others).  Returns the
 // number of deviations written; lane 0's top is the first of them.
 __device__ __forceinline__ int write_short_row(const SfxtParams& p, int rb, bool valid,
                                                const DevSidetrack& rec, DevSidetrack& top) {
