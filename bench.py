@@ -56,9 +56,9 @@ METRIC = "K-paths/sec"
 # DRAM bytes (read + write) per query of the dominant kernels on this
 # workload, from the one-pass ncu capture summarised in
 # profiles/sfxt_dataflow_kernel_large400k.md (the suffix-tree build does not
-# depend on K; the engine's figure is its two launches at K = 1e6).
-KERNEL_TRAFFIC = {"sfxt_dataflow_kernel": 708_980_736 + 625_738_752,
-                  "engine_kernel": 757_760 + 102_573_056 + 188_904_960}
+# depend on K; the engine's figure is its block and grid launches at K = 1e6).
+KERNEL_TRAFFIC = {"sfxt_dataflow_kernel": 724_916_736 + 633_657_600,
+                  "engine_kernel": 1_389_568 + 174_598_912 + 237_775_616}
 
 
 def peaks():
