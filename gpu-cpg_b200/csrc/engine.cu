@@ -1464,6 +1464,12 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
     for (int r = 0;; ++r, ++rounds) {
       const unsigned n = s_front[r % 3];
       if (n == 0) break;
+      // the counter goes past the end when put() dropped items: nothing behind
+      // the end is read
+      if (n > kBlkFront + front_gcap) {
+        if (tid == 0) eng_fail(p, kDevCapacity);
+        break;
+      }
       // (last round's counter, the next round's; nobody reads or adds to it now)
       if (tid == 0) s_front[(r + 2) % 3] = 0;
       if (!own) {

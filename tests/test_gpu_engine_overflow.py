@@ -1,0 +1,79 @@
+"""Queries that outgrow what their block of the engine holds: more tied roots
+than frontier slots, against the oracle.  The overflow is detected, nothing
+behind the end is read, and the handle answers other queries afterwards."""
+import numpy as np
+import pytest
+
+import cpg_b200
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def tied_roots(n_src):
+    """n_src sources with one unit edge each into one sink: every path costs 1."""
+    src = np.arange(n_src, dtype=np.int32)
+    return n_src + 1, src, np.full(n_src, n_src, np.int32), np.ones(n_src, np.float32)
+
+
+def generated(seed, n_pins=2000, weight_kind=0):
+    d = cpg_b200.generate(cpg_b200.gen_params(
+        seed=seed, n_pins=n_pins, n_levels=20, n_first=8, n_last=8, level_span=3, degree_kind=0,
+        deg_lo=1, deg_hi=5, weight_kind=weight_kind, iw_lo=1, iw_hi=9, add_virtual=1))
+    return d.n, d.src, d.dst, d.w
+
+
+def expected(graph, k, ref_roots):
+    return oracle.OracleGraph.from_edges(*graph).closure_topk(k, ref_roots=ref_roots)[0]["slack"]
+
+
+def bits_equal(a, b):
+    return np.array_equal(np.asarray(a, np.float32).view(np.uint32),
+                          np.asarray(b, np.float32).view(np.uint32))
+
+
+def dag_of(graph):
+    n, src, dst, w = graph
+    return cpg_b200.Dag(n, src, dst, w)
+
+
+def run_batch(graphs, gi, ks, root_seeding, engine_ctas=0):
+    """Costs of the queries and the batch's statistics."""
+    if engine_ctas:
+        b = cpg_b200.Batch.__new__(cpg_b200.Batch)
+        o = cpg_b200.Options()
+        cpg_b200.lib.cpg_options_init(cpg_b200.C.byref(o))
+        o.division, o.root_seeding, o.engine_ctas = cpg_b200.DIV_IEEE, root_seeding, engine_ctas
+        b._b, b.ks = cpg_b200.C.c_void_p(), []
+        assert cpg_b200.lib.cpg_batch_create(cpg_b200.C.byref(b._b), cpg_b200.C.byref(o)) == 0
+    else:
+        b = cpg_b200.Batch(division=cpg_b200.DIV_IEEE, root_seeding=root_seeding)
+    with b:
+        for g in graphs:
+            b.add_dag(dag_of(g))
+        b.commit()
+        b.set_queries(gi, ks)
+        b.run()
+        return [b.costs(q) for q in range(len(ks))], b.stats()
+
+
+@pytest.mark.parametrize("n_src,k", [(67072, 1), (67073, 1), (100_000, 1), (100_000, 3000),
+                                     (150_000, 4096), (150_000, 4097)])
+def test_more_tied_roots_than_frontier_slots(n_src, k):
+    with cpg_b200.CpGen(division=cpg_b200.DIV_IEEE, root_seeding=cpg_b200.ROOTS_ALL) as g:
+        g.load_edges(*tied_roots(n_src))
+        g.report_paths(k)
+        assert bits_equal(g.get_slacks(k), np.ones(k, np.float32))
+        g.load_edges(*generated(5))
+        g.report_paths(500)
+        assert bits_equal(g.get_slacks(500), expected(generated(5), 500, 0))
+
+
+def test_tied_roots_of_a_small_query_beside_large_ones():
+    graphs = [tied_roots(100_000), generated(6), generated(7, weight_kind=1)]
+    gi, ks = [0, 1, 2, 1], [1, 20_000, 16_000, 3]
+    got, _ = run_batch(graphs, gi, ks, cpg_b200.ROOTS_ALL)
+    want = [expected(g, max(ks), 0) for g in graphs[1:]]
+    assert bits_equal(got[0], [1.0])
+    for q in (1, 2, 3):
+        assert bits_equal(got[q], want[gi[q] - 1][:ks[q]]), q
