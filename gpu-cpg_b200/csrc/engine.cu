@@ -959,6 +959,14 @@ __device__ void next_phase(const EngineParams& p, int phase, bool finish) {
   }
 }
 
+// Slots of the path store in use.  The blocks reserve slots in chunks, whose
+// last may go past the end of the store with only its used part inside; a path
+// without a slot fails the launch where it is made (grow_path).
+__device__ __forceinline__ unsigned long long stored_paths(const EngineParams& p) {
+  const unsigned long long n = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->paths);
+  return n < p.ps.cap ? n : p.ps.cap;
+}
+
 // ------------------------------------------------------------------ kernel
 __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
   const unsigned long long tid =
@@ -976,7 +984,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
   int pin = 0;
   const int phase0 = __ldcg(&p.ctr->res_phase);
   unsigned long long n_pend = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->pend_out);
-  unsigned long long n_paths = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->paths);
+  unsigned long long n_paths = stored_paths(p);
   STAMP(0);
 
   for (int phase = phase0;; ++phase) {
@@ -1041,16 +1049,12 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
     if (!eng_sync_last(p, [&]() { next_phase(p, phase, true); }))
       return;
     STAMP(1);
-    n_paths = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->paths);
+    n_paths = stored_paths(p);
     n_pend = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->pend_out);
     pin ^= 1;
   }
 
   // ---------------------------------------------------------------- output
-  if (n_paths > p.ps.cap) {
-    eng_fail(p, kDevCapacity);
-    return;
-  }
   for (unsigned long long i = tid; i < n_paths; i += nth) p.rank_of[i] = -1;
   // One query: once K non-zero paths were accepted, the final phase's split
   // T is the K-th cost of the paths and pending items then known, and every

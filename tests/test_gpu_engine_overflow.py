@@ -1,6 +1,7 @@
 """Queries that outgrow what their block of the engine holds: more tied roots
-than frontier slots, against the oracle.  The overflow is detected, nothing
-behind the end is read, and the handle answers other queries afterwards."""
+than frontier slots, path slots reserved past the end of the store, against
+the oracle.  The overflow is detected, nothing behind the end is read, and the
+handle answers other queries afterwards."""
 import numpy as np
 import pytest
 
@@ -77,3 +78,14 @@ def test_tied_roots_of_a_small_query_beside_large_ones():
     assert bits_equal(got[0], [1.0])
     for q in (1, 2, 3):
         assert bits_equal(got[q], want[gi[q] - 1][:ks[q]]), q
+
+
+@pytest.mark.parametrize("queries", [256, 257, 600])
+def test_small_queries_of_the_grid_launch_reserve_past_the_path_store(queries):
+    # a store of 65,536 slots and the graph's source, and 256 slots a query
+    graphs = [generated(8)]
+    want = expected(graphs[0], 40, 0)
+    ks = [1 + q % 40 if queries == 600 else 1 for q in range(queries)]
+    got, _ = run_batch(graphs, [0] * queries, ks, cpg_b200.ROOTS_ALL, engine_ctas=8)
+    for q in range(queries):
+        assert bits_equal(got[q], want[:ks[q]]), q
