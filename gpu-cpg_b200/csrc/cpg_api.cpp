@@ -121,10 +121,10 @@ struct cpg_handle {
   int sfxt_grid_limit = 0;
   int engine_grid_limit = 0;
   int sel_schedule = 0;  // 0: 11/11/10-bit select digits, 1: 8/8/8/8
-  // the prepared queries: whether any goes on to the grid launch, and the
-  // grid's part of the path store and the piles
+  // the prepared queries: whether any goes on to the grid launch for sure, and
+  // the part of the path store and the pending pile its items are left in
   bool engine_grid_part = false;
-  unsigned long long grid_paths = 0, grid_pend = 0, grid_front = 0;
+  unsigned long long left_paths = 0, left_pend = 0;
 
   // staging
   void* pinned = nullptr;
@@ -1070,13 +1070,15 @@ int try_query(cpg_handle* h, unsigned long long k) {
 // finish (read counters back, map errors).
 
 // Which queries their blocks answer whole, where each query's costs go, and
-// every block's share of the path store and piles: in proportion to k, the
-// queries that go on to the grid launch first, so that the grid's part of
-// each is one range from 0.
+// every block's share of the path store and piles, the queries that go on to
+// the grid launch first, so that what they leave lies in one range from 0.  A
+// share follows k up to what a block answers, and the constant part is for small queries, whose
+// growth phases overshoot k by more: among 48 of k up to 50,000 one of
+// k = 2,554 had 25,400 items pending and outgrew 8 k and the block's own 4,096.
 void engine_layout(cpg_handle* h, std::vector<EngineQuery>& qs) {
   const long long whole_max = h->opts.engine_ctas > 0 ? 0 : qs.size() > 1 ? kWholeBeside : kWholeAlone;
   auto weight = [](const EngineQuery& q) {
-    return static_cast<unsigned long long>(std::max<long long>(q.k, 64)) +
+    return static_cast<unsigned long long>(std::min<long long>(q.k, kBlockMaxK)) + 2048 +
            static_cast<unsigned long long>(q.src_end - q.src_beg);
   };
   unsigned long long all = 0, off = 0, at = 0;
@@ -1104,9 +1106,8 @@ void engine_layout(cpg_handle* h, std::vector<EngineQuery>& qs) {
       if (!whole) h->engine_grid_part = true;
     }
     if (!whole) {
-      h->grid_paths = part(h->cap_paths, at);
-      h->grid_pend = part(h->cap_pend, at);
-      h->grid_front = part(h->cap_front, at);
+      h->left_paths = part(h->cap_paths, at);
+      h->left_pend = part(h->cap_pend, at);
     }
   }
 }
@@ -1138,21 +1139,7 @@ Status engine_prepare(cpg_handle* h, std::vector<EngineQuery> qs, unsigned long 
   return CPG_OK;
 }
 
-// One launch with a block per query, then, unless the blocks answer every
-// query whole, the grid launch on the handle's CTA count, which goes on with
-// what they left.  *launches receives the number of launches.
-Status engine_enqueue(cpg_handle* h, int nq, unsigned long long k_total,
-                      int* launches = nullptr) {
-  cudaStream_t s = h->stream;
-  int grid = 0;
-  CK(engine_grid(h->device, h->engine_grid_limit, &grid), "engine occupancy");
-  CK(cudaMemsetAsync(h->d_ectr.p, 0, sizeof(EngineCounters), s), "memset");
-  if (h->engine_grid_part) {
-    CK(cudaMemsetAsync(h->d_ehist.p, 0, static_cast<size_t>(nq) * kSelBins * 4, s), "memset");
-    // every output slot is written by the compaction; zero-filling keeps a path
-    // index in range even if selection and compaction ever disagreed
-    CK(cudaMemsetAsync(h->d_vals.p, 0, 2 * k_total * 4, s), "memset");
-  }
+EngineParams engine_params(cpg_handle* h, int nq, unsigned long long k_total, int grid) {
   EngineParams p{};
   p.g.adjp = P<int32_t>(h->d_adjp);
   p.g.dist = P<int32_t>(h->d_dist);
@@ -1166,14 +1153,15 @@ Status engine_enqueue(cpg_handle* h, int nq, unsigned long long k_total,
   p.nq = nq;
   p.root_ref = h->opts.root_seeding == CPG_ROOTS_REFERENCE;
   p.ps = path_store(h);
-  p.ps.cap = h->grid_paths;
   p.pq = P<int32_t>(h->d_pq);
   p.pend[0] = P<Item>(h->d_pend0);
   p.pend[1] = P<Item>(h->d_pend1);
-  p.pend_cap = h->grid_pend;
+  p.pend_cap = h->cap_pend;
+  p.left_pend = h->left_pend;
+  p.left_paths = h->left_paths;
   p.front[0] = P<Item>(h->d_front0);
   p.front[1] = P<Item>(h->d_front1);
-  p.front_cap = h->grid_front;
+  p.front_cap = h->cap_front;
   p.hist = P<unsigned int>(h->d_ehist);
   p.keys[0] = P<unsigned int>(h->d_keys);
   p.keys[1] = P<unsigned int>(h->d_keys) + k_total;
@@ -1205,27 +1193,71 @@ Status engine_enqueue(cpg_handle* h, int nq, unsigned long long k_total,
     p.sel_shift[2] = 0;  p.sel_bits[2] = 10;
   }
   p.solo_stop = kEngSoloStop;
+  return p;
+}
+
+// The grid launch on the handle's CTA count, which goes on with what the
+// blocks left.
+Status engine_enqueue_grid(cpg_handle* h, const EngineParams& p, unsigned long long k_total) {
+  cudaStream_t s = h->stream;
+  CK(cudaMemsetAsync(h->d_ehist.p, 0, static_cast<size_t>(p.nq) * kSelBins * 4, s), "memset");
+  // every output slot is written by the compaction; zero-filling keeps a path
+  // index in range even if selection and compaction ever disagreed
+  CK(cudaMemsetAsync(h->d_vals.p, 0, 2 * k_total * 4, s), "memset");
+  CK(launch_engine(p, h->device, s), "engine launch");
+  return CPG_OK;
+}
+
+// One launch with a block per query, then the grid launch if a query is known
+// to need it; engine_finish launches it for one that outgrew its block.
+// *launches receives the number of launches.
+Status engine_enqueue(cpg_handle* h, int nq, unsigned long long k_total,
+                      int* launches = nullptr) {
+  cudaStream_t s = h->stream;
+  int grid = 0;
+  CK(engine_grid(h->device, h->engine_grid_limit, &grid), "engine occupancy");
+  CK(cudaMemsetAsync(h->d_ectr.p, 0, sizeof(EngineCounters), s), "memset");
+  const EngineParams p = engine_params(h, nq, k_total, grid);
   CK(launch_engine_blocks(p, s), "engine launch");
-  if (h->engine_grid_part) CK(launch_engine(p, h->device, s), "engine launch");
+  if (h->engine_grid_part) {
+    const Status st = engine_enqueue_grid(h, p, k_total);
+    if (st != CPG_OK) return st;
+  }
   if (launches) *launches = h->engine_grid_part ? 2 : 1;
   return CPG_OK;
 }
 
-// Counters and the per-query table back on the host.  kRetry on overflow.
+// Counters and the per-query table back on the host, after the grid launch if
+// a query turned out to need it (`done` is recorded again behind that).
+// kRetry on overflow.
 int engine_finish(cpg_handle* h, std::vector<EngineQuery>& qout, EngineCounters& c,
-                  unsigned long long k_total) {
+                  unsigned long long k_total, cudaEvent_t done) {
   const size_t nq = qout.size();
   char* hb = static_cast<char*>(h->pinned);
   // a few queries' table comes back with the counters, in one pinned copy
   constexpr size_t kQoff = (sizeof(EngineCounters) + 127) & ~size_t{127};
   const bool inline_q = kQoff + nq * sizeof(EngineQuery) <= kPinnedBytes;
-  CK(cudaMemcpyAsync(hb, h->d_ectr.p, sizeof(EngineCounters), cudaMemcpyDeviceToHost,
-                     h->stream), "D2H counters");
-  if (inline_q)
-    CK(cudaMemcpyAsync(hb + kQoff, h->d_equery.p, nq * sizeof(EngineQuery),
-                       cudaMemcpyDeviceToHost, h->stream), "D2H queries");
-  CK(cudaStreamSynchronize(h->stream), "engine");
-  std::memcpy(&c, hb, sizeof(c));
+  for (int pass = 0; pass < 2; ++pass) {
+    CK(cudaMemcpyAsync(hb, h->d_ectr.p, sizeof(EngineCounters), cudaMemcpyDeviceToHost,
+                       h->stream), "D2H counters");
+    if (inline_q)
+      CK(cudaMemcpyAsync(hb + kQoff, h->d_equery.p, nq * sizeof(EngineQuery),
+                         cudaMemcpyDeviceToHost, h->stream), "D2H queries");
+    CK(cudaStreamSynchronize(h->stream), "engine");
+    std::memcpy(&c, hb, sizeof(c));
+    if (pass == 1 || c.err != kDevOk || !c.stopped || (h->engine_grid_part && !c.restarts)) break;
+    int grid = 0;
+    CK(engine_grid(h->device, h->engine_grid_limit, &grid), "engine occupancy");
+    const EngineParams p = engine_params(h, static_cast<int>(nq), k_total, grid);
+    if (c.restarts) {
+      CK(launch_seed_left(p, h->stream), "engine launch");
+      h->stats.kernel_launches += 1;
+    }
+    const Status st = engine_enqueue_grid(h, p, k_total);
+    if (st != CPG_OK) return st;
+    CK(cudaEventRecord(done, h->stream), "event");
+    h->stats.kernel_launches += 1;
+  }
   if (c.err == kDevTimeout)
     return fail(h, CPG_ERR_TIMEOUT, "query engine: grid barrier wait ran out");
   if (c.err == kDevCapacity) {
@@ -1239,7 +1271,7 @@ int engine_finish(cpg_handle* h, std::vector<EngineQuery>& qout, EngineCounters&
   else
     CK(cudaMemcpy(qout.data(), h->d_equery.p, nq * sizeof(EngineQuery), cudaMemcpyDeviceToHost),
        "D2H queries");
-  c.paths += c.blk_paths;
+  c.paths = c.paths + c.blk_paths - c.blk_pad;
   c.pend_out += c.blk_pend;
   h->stats.paths_accepted = static_cast<int64_t>(c.paths);
   h->stats.items_generated = static_cast<int64_t>(c.paths + c.pend_out);
@@ -1278,7 +1310,7 @@ int engine_query(cpg_handle* h, unsigned long long k) {
   CK(cudaEventRecord(h->ev[3], s), "event");
   h->stats.kernel_launches += launches;
   EngineCounters c;
-  const int r = engine_finish(h, qs, c, k);
+  const int r = engine_finish(h, qs, c, k, h->ev[3]);
   if (r != CPG_OK) return r;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, h->ev[2], h->ev[3]);
@@ -1991,7 +2023,7 @@ int batch_step(cpg_batch* b, bool rebuild) {
   }
   b->qout = b->qs;
   EngineCounters c;
-  const int r = engine_finish(h, b->qout, c, b->k_total);
+  const int r = engine_finish(h, b->qout, c, b->k_total, h->ev[5]);
   if (r == kRetry) {
     b->prepared = false;
     return kRetry;
@@ -2372,7 +2404,7 @@ int server_launch(cpg_server* sv, const std::vector<ServerReq>& batch,
   if (st != CPG_OK) return st;
   CK(cudaEventRecord(h->ev[5], s), "event");
   EngineCounters c;
-  const int r = engine_finish(h, qs, c, k_total);
+  const int r = engine_finish(h, qs, c, k_total, h->ev[5]);
   if (r != CPG_OK) return r;
   float ms = 0.f;
   cudaEventElapsedTime(&ms, h->ev[4], h->ev[5]);

@@ -390,6 +390,10 @@ constexpr int kJBits = 20;          // ... and the deviation index in 20 bits
 constexpr unsigned kJMask = (1u << kJBits) - 1u;
 constexpr int kSelBins = 2048;
 
+// What a query's block left to the grid launch: nothing, its pending items (and
+// the paths accepted so far), or the whole query, which outgrew the block.
+enum EngineLeft : int { kAnswered = 0, kLeftItems = 1, kLeftRoots = 2 };
+
 struct EngineQuery {
   long long k;
   int src_beg, src_end;       // this query's sources in EngineParams::srcs
@@ -405,10 +409,11 @@ struct EngineQuery {
   unsigned long long k_out, out_off, out_lt, out_eq;
   int phases;
   int whole;                  // answered by its own block (engine_block_kernel)
+  int left;                   // set by the block: EngineLeft
   // the last growth phase: accepted before it, promoted, of how many pending
   unsigned long long acc_prev, last_j, last_pend;
-  // set by the host: where the query's costs go, and its block's share of the
-  // path store and of the global overflow of its piles
+  // set by the host: its block's share of the path store, and of the piles for
+  // what its own do not hold
   unsigned long long path_base, path_cap, pend_base, pend_cap, front_base, front_cap;
   unsigned long long seg_off;  // the grid's output: its segment of the sorted paths
 };
@@ -433,7 +438,11 @@ struct EngineCounters {
   int sorted_buf;             // which vals[] holds the sorted path indices
   int stopped;                // a block left its query to the grid launch
   int res_phase;              // ... after this many phases at most
-  unsigned long long blk_paths, blk_pend;  // paths and pending items of the whole queries
+  int res_pin;                // ... its pending items in this pile
+  int restarts;               // a query outgrew its block and waits for seed_left_kernel
+  // paths and pending items of the queries the blocks answered, and slots the
+  // others reserved that hold no path
+  unsigned long long blk_paths, blk_pend, blk_pad;
   // device time per stage (ns): 0 seed, 1 decide/bookkeeping, 2 select,
   // 3 promote, 4 closure, 5 output select, 6 output sort, 7 emit
   unsigned long long t_ns[8];
@@ -450,6 +459,8 @@ struct EngineParams {
   int32_t* pq;                // query of each accepted path
   Item* pend[2];
   unsigned long long pend_cap;
+  // the part of pend[0] and of the path store that blocks leave items and paths in
+  unsigned long long left_pend, left_paths;
   Item* front[2];
   unsigned long long front_cap;
   unsigned int* hist;         // nq * kSelBins
@@ -478,6 +489,8 @@ struct EngineParams {
 // host sizes sort_hist as 256 * grid) for a given CTA limit (0: maximum).
 int engine_grid(int device, int limit, int* grid_out);
 int launch_engine(const EngineParams& p, int device, void* stream);
+// Seeds the queries that outgrew their blocks, before the launch above.
+int launch_seed_left(const EngineParams& p, void* stream);
 // One block per query: runs `whole` queries to the end and the others' first
 // phases (engine_block_kernel).
 int launch_engine_blocks(const EngineParams& p, void* stream);

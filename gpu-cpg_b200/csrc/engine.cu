@@ -940,6 +940,8 @@ __device__ bool decide_query(const EngineParams& p, EngineQuery& Q) {
 __device__ void next_phase(const EngineParams& p, int phase, bool finish) {
   if (threadIdx.x == 0) {
     if (finish) p.ctr->phases = phase + 1;
+    // (the blocks' last chunk may end behind their part of the store)
+    else if (p.nq > 1 && p.ctr->paths > p.left_paths) p.ctr->paths = p.left_paths;
     p.ctr->active = 0;
     p.ctr->sel_paths = 0;
     p.ctr->sel_stop = 0;
@@ -959,9 +961,8 @@ __device__ void next_phase(const EngineParams& p, int phase, bool finish) {
   }
 }
 
-// Slots of the path store in use.  The blocks reserve slots in chunks, whose
-// last may go past the end of the store with only its used part inside; a path
-// without a slot fails the launch where it is made (grow_path).
+// Slots of the path store in use.  (The counter goes past the end when paths
+// found no slot, which fails the launch where they are made, grow_path.)
 __device__ __forceinline__ unsigned long long stored_paths(const EngineParams& p) {
   const unsigned long long n = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->paths);
   return n < p.ps.cap ? n : p.ps.cap;
@@ -976,12 +977,14 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
   if (threadIdx.x == 0) s_stage = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) t_last = gtime();
   // the blocks (engine_block_kernel) ran every query's first phases; what
-  // they left to the grid is in pile 0.  An error there ends this launch too.
+  // they left to the grid is in pile res_pin.  Nothing to do, or a query that
+  // outgrew its block and is not seeded again yet, ends this launch.
   if (*reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk ||
-      !*reinterpret_cast<volatile int*>(&p.ctr->stopped))
+      !*reinterpret_cast<volatile int*>(&p.ctr->stopped) ||
+      *reinterpret_cast<volatile int*>(&p.ctr->restarts))
     return;
   if (!eng_sync_last(p, [&]() { next_phase(p, 0, false); })) return;
-  int pin = 0;
+  int pin = __ldcg(&p.ctr->res_pin);
   const int phase0 = __ldcg(&p.ctr->res_phase);
   unsigned long long n_pend = *reinterpret_cast<volatile unsigned long long*>(&p.ctr->pend_out);
   unsigned long long n_paths = stored_paths(p);
@@ -1136,7 +1139,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
     ENG_SYNC();
     for (unsigned long long qi = tid; qi < static_cast<unsigned long long>(p.nq); qi += nth) {
       EngineQuery& Q = p.q[qi];
-      if (Q.whole) {  // its block wrote its output
+      if (Q.left == kAnswered) {  // its block wrote its output
         Q.mode = 0;
         continue;
       }
@@ -1152,7 +1155,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       unsigned long long acc = 0;
       for (int qi = 0; qi < p.nq; ++qi) {
-        if (p.q[qi].whole) continue;
+        if (p.q[qi].left == kAnswered) continue;
         p.q[qi].seg_off = acc;
         acc += p.q[qi].k_out;
       }
@@ -1276,7 +1279,14 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
 // one is left to the grid launch at the top of a phase with more than
 // solo_stop items pending.  Blocks never wait on one another, so any number
 // of queries run in one ordinary launch, as many at a time as there are SMs.
+//
+// A block's part of the path store and of the piles is a share.  A query that
+// outgrows it is given to the grid launch, which starts it again from its roots
+// with all of the piles, and of the store but for the paths left there: what a
+// launch cannot answer, and what it asks for then, depends on all of its
+// queries together, not on a share.
 constexpr unsigned kBlkPend = 4096, kBlkFront = 1536;
+constexpr int kChunks = 64;  // path chunks of a query that leaves its paths
 
 struct BlockMem {
   Item pend[2][kBlkPend];
@@ -1294,10 +1304,12 @@ struct BlkPile {
   __device__ __forceinline__ Item get(unsigned i) const {
     return i < scap ? s[i] : load_item(g, i - scap);
   }
-  __device__ __forceinline__ void put(const EngineParams& p, unsigned i, const Item& it) const {
+  // false: past the end, not stored
+  __device__ __forceinline__ bool put(unsigned i, const Item& it) const {
     if (i < scap) s[i] = it;
     else if (i - scap < gcap) g[i - scap] = it;
-    else eng_fail(p, kDevCapacity);
+    else return false;
+    return true;
   }
 };
 
@@ -1364,13 +1376,24 @@ __device__ void blk_sort(unsigned long long* a, unsigned n2) {
   }
 }
 
+// Slots [beg, end) of the path store that hold no path of an answer: costs of
+// zero, which no step counts (threads t, t + nt, ...).
+__device__ void clear_slots(const EngineParams& p, int qi, unsigned long long beg,
+                            unsigned long long end, unsigned t, unsigned nt) {
+  if (end > p.left_paths) end = p.left_paths;
+  for (unsigned long long x = beg + t; x < end; x += nt) {
+    p.ps.cost[x] = 0.f;
+    p.pq[x] = qi;
+  }
+}
+
 __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams p) {
   extern __shared__ __align__(16) unsigned char blk_raw[];
   BlockMem& m = *reinterpret_cast<BlockMem*>(blk_raw);
   __shared__ EngineQuery Q;
   __shared__ unsigned s_pend[2], s_front[3], s_nz, s_pnz, s_chosen, s_take[2];
-  __shared__ unsigned long long s_base, s_chunk[2];
-  __shared__ int s_go;
+  __shared__ unsigned long long s_base, s_chunk[2], s_list[kChunks][2];
+  __shared__ int s_go, s_fits, s_chunks;
   const int qi = blockIdx.x;
   const unsigned q = static_cast<unsigned>(qi);
   const unsigned tid = threadIdx.x, nth = blockDim.x;
@@ -1379,44 +1402,49 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
   if (tid == 0) {
     s_stage = 0;
     Q = p.q[qi];
+    Q.left = kAnswered;
     s_pend[0] = s_pend[1] = 0;
     s_chunk[0] = s_chunk[1] = 0;
+    s_chunks = 0;
   }
   for (int i = tid; i < kSelBins; i += nth) m.hist[i] = 0;  // every pick leaves it zero again
   __syncthreads();
   const bool whole = Q.whole != 0;
   // this query's paths: a share of its own, or (several queries, not whole)
   // chunks of the store the grid launch goes on with
-  const bool own = whole || p.nq == 1;
-  const unsigned long long path_cap = own ? Q.path_base + Q.path_cap : p.ps.cap;
-  Item* const g0 = (whole ? p.pend[0] : p.pend[1]) + Q.pend_base;
-  Item* const g1 = p.pend[1] + Q.pend_base + (whole ? 0 : Q.pend_cap / 2);
-  const unsigned long long pend_gcap = whole ? Q.pend_cap : Q.pend_cap / 2;
-  const unsigned long long front_base = Q.front_base, front_gcap = Q.front_cap;
+  const bool alone = p.nq == 1, own = whole || alone;
+  // where the piles spill to: its shares; a query that leaves items for the
+  // grid in pile 0 beside others has two halves of its share of pile 1
+  Item* const g0 = (own ? p.pend[0] : p.pend[1]) + Q.pend_base;
+  Item* const g1 = p.pend[1] + Q.pend_base + (own ? 0 : Q.pend_cap / 2);
+  const unsigned long long pend_gcap = own ? Q.pend_cap : Q.pend_cap / 2;
   auto pend_pile = [&](int b) { return BlkPile{m.pend[b], b ? g1 : g0, kBlkPend, pend_gcap}; };
   auto front_pile = [&](int b) {
-    return BlkPile{m.front[b], p.front[b] + front_base, kBlkFront, front_gcap};
+    return BlkPile{m.front[b], p.front[b] + Q.front_base, kBlkFront, Q.front_cap};
   };
-  if (tid < 32)
+  // `over`: this thread met the end of a share (more sources than the pile
+  // holds are not even seeded).  outgrown: some thread did, known to all;
+  // nothing behind an end is read after it.
+  bool over = static_cast<unsigned>(Q.src_end - Q.src_beg) > kBlkPend + pend_gcap;
+  if (tid < 32 && !over)
     seed_query(p, qi, Q, [&](bool keep, const Item& it) {
       const unsigned slot = blk_append(&s_pend[0], keep);
-      if (keep) pend_pile(0).put(p, slot, it);
+      if (keep) over |= !pend_pile(0).put(slot, it);
     });
-  __syncthreads();
+  bool outgrown = __syncthreads_or(over);
   STAMP(0);
 
   int pin = 0, phase = 0, rounds = 0;
   unsigned n_paths = 0;  // of an `own` query: slots path_base ..
-  for (;; ++phase) {
+  for (; !outgrown; ++phase) {
     const unsigned n_pend = s_pend[pin];
     __syncthreads();
     if (tid == 0) {
       // (paths in chunks: the final phase, which selects over them, is the
       // grid's)
       const bool stay = whole || (n_pend <= p.solo_stop &&
-                                  (own || Q.paths_nz < static_cast<unsigned long long>(Q.k)));
-      s_go = *reinterpret_cast<volatile int*>(&p.ctr->err) == kDevOk && stay &&
-             decide_query(p, Q);
+                                  (alone || Q.paths_nz < static_cast<unsigned long long>(Q.k)));
+      s_go = stay && decide_query(p, Q);
       s_pend[pin ^ 1] = 0;
       s_front[0] = s_front[1] = s_front[2] = 0;
       s_nz = s_pnz = 0;
@@ -1457,37 +1485,32 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
       const bool take = on && it.cost <= lim, keep = on && !take;
       const unsigned a = blk_append(&s_front[0], take);
       const unsigned b = blk_append(&s_pend[pin ^ 1], keep);
-      if (take) front_pile(0).put(p, a, it);
-      if (keep) next.put(p, b, it);
+      if (take) over |= !front_pile(0).put(a, it);
+      if (keep) over |= !next.put(b, it);
       acc_pnz += keep && it.cost != 0.0f;
     }
-    __syncthreads();
+    outgrown = __syncthreads_or(over);
     STAMP(3);
     // closure
     unsigned acc_nz = 0;
-    for (int r = 0;; ++r, ++rounds) {
+    for (int r = 0; !outgrown; ++r, ++rounds) {
       const unsigned n = s_front[r % 3];
       if (n == 0) break;
-      // the counter goes past the end when put() dropped items: nothing behind
-      // the end is read
-      if (n > kBlkFront + front_gcap) {
-        if (tid == 0) eng_fail(p, kDevCapacity);
-        break;
-      }
       // (last round's counter, the next round's; nobody reads or adds to it now)
       if (tid == 0) s_front[(r + 2) % 3] = 0;
       if (!own) {
-        // n slots in a row; what a chunk leaves over is filled with zero
-        // costs, which no later step counts
+        // n slots in a row; what a chunk leaves over holds no path
         if (tid == 0) {
           if (s_chunk[0] + n > s_chunk[1]) {
-            for (unsigned long long x = s_chunk[0]; x < s_chunk[1] && x < p.ps.cap; ++x) {
-              p.ps.cost[x] = 0.f;
-              p.pq[x] = qi;
-            }
-            const unsigned grab = n > 256 ? n : 256;
-            s_chunk[0] = atomicAdd(&p.ctr->paths, static_cast<unsigned long long>(grab));
+            clear_slots(p, qi, s_chunk[0], s_chunk[1], 0, 1);
+            // (the first chunks of all queries fit a quarter of the store)
+            unsigned long long grab = p.left_paths / (4ull * static_cast<unsigned long long>(p.nq));
+            grab = max(min(grab, 256ull), static_cast<unsigned long long>(max(n, n_paths / 4)));
+            s_chunk[0] = atomicAdd(&p.ctr->paths, grab);
             s_chunk[1] = s_chunk[0] + grab;
+            s_list[s_chunks][0] = s_chunk[0];
+            s_list[s_chunks][1] = s_chunk[1];
+            ++s_chunks;
           }
           s_base = s_chunk[0];
           s_chunk[0] += n;
@@ -1495,6 +1518,11 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
         __syncthreads();
       }
       const unsigned long long base = own ? Q.path_base + n_paths : s_base;
+      // (the same for every thread)
+      if (own ? n_paths + n > Q.path_cap : base + n > p.left_paths || s_chunks == kChunks) {
+        outgrown = true;
+        break;
+      }
       const BlkPile in = front_pile(r & 1), out = front_pile((r + 1) & 1);
       for (unsigned i0 = tid & ~31u; i0 < n; i0 += nth) {
         const unsigned i = i0 + (tid & 31);
@@ -1505,7 +1533,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
         it.j = 0;
         if (i < n) it = in.get(i);
         const unsigned long long qp = base + i;
-        const Grown g = grow_path(p, it, i < n, q, qp, path_cap, lim, tie);
+        const Grown g = grow_path(p, it, i < n, q, qp, ~0ull, lim, tie);
         acc_nz += g.stored && it.cost != 0.0f;
         acc_pnz += pending_nz(g);
         unsigned bt = blk_reserve(&s_front[(r + 1) % 3], __popc(g.tm));
@@ -1515,13 +1543,12 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
           const unsigned bit = 1u << k;
           if (!((g.tm | g.dm) & bit)) continue;
           const Item c = child_of(g, it, q, qp, k);
-          if (g.tm & bit) out.put(p, bt++, c);
-          else next.put(p, bd++, c);
+          if (g.tm & bit) over |= !out.put(bt++, c);
+          else over |= !next.put(bd++, c);
         }
       }
       n_paths += n;
-      if (__syncthreads_or(tid == 0 && *reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk))
-        break;
+      outgrown = __syncthreads_or(over);
     }
     acc_nz = __reduce_add_sync(0xffffffffu, acc_nz);
     acc_pnz = __reduce_add_sync(0xffffffffu, acc_pnz);
@@ -1547,33 +1574,57 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
     atomicMax(&p.ctr->res_phase, phase);
     atomicMax(&p.ctr->phases, phase);
     atomicAdd(&p.ctr->rounds, rounds);
+    if (!whole && !outgrown) {
+      // room for the pending items in the pile the grid launch starts from
+      unsigned long long at = 0, seen;
+      do {
+        seen = at;
+        s_fits = seen + n_pend <= p.left_pend;
+        if (s_fits) at = atomicCAS(&p.ctr->pend_out, seen, seen + n_pend);
+      } while (s_fits && at != seen);
+      s_base = seen;
+    }
   }
-  if (__syncthreads_or(tid == 0 && *reinterpret_cast<volatile int*>(&p.ctr->err) != kDevOk))
-    return;
-  if (!whole) {
-    // the rest is the grid's: the pending items join pile 0 and the next
-    // phase is decided there
+  __syncthreads();
+  if (!whole && !outgrown) outgrown = !s_fits;
+  if (!own) {
+    // slots without a path; the paths of a query that starts again are no part
+    // of the answer
+    if (!outgrown) clear_slots(p, qi, s_chunk[0], s_chunk[1], tid, nth);
+    unsigned long long slots = 0;
+    for (int c = 0; c < s_chunks; ++c) {
+      if (outgrown) clear_slots(p, qi, s_list[c][0], s_list[c][1], tid, nth);
+      slots += min(s_list[c][1], p.left_paths) - min(s_list[c][0], p.left_paths);
+    }
+    if (tid == 0) atomicAdd(&p.ctr->blk_pad, slots - (outgrown ? 0 : n_paths));
+  }
+  if (outgrown) {
     if (tid == 0) {
-      if (own) {
-        p.ctr->paths = n_paths;
-      } else {
-        for (unsigned long long x = s_chunk[0]; x < s_chunk[1] && x < p.ps.cap; ++x) {
-          p.ps.cost[x] = 0.f;
-          p.pq[x] = qi;
-        }
-      }
       Q.mode = 0;
-      s_base = atomicAdd(&p.ctr->pend_out, static_cast<unsigned long long>(n_pend));
+      Q.left = kLeftRoots;
+      p.q[qi] = Q;
+      p.ctr->restarts = 1;
       p.ctr->stopped = 1;
     }
-    __syncthreads();
+    return;
+  }
+  if (!whole) {
+    // the rest is the grid's, which decides the next phase.  (A query alone
+    // spilled into the very pile: its other items join behind those.)
+    const unsigned spilled = alone && n_pend > kBlkPend ? n_pend - kBlkPend : 0;
     const BlkPile left = pend_pile(pin);
-    for (unsigned i = tid; i < n_pend; i += nth) {
-      if (s_base + i < p.pend_cap) p.pend[0][s_base + i] = left.get(i);
-      else eng_fail(p, kDevCapacity);
+    Item* const to = p.pend[alone ? pin : 0] + (alone ? spilled : s_base);
+    for (unsigned i = tid; i < n_pend - spilled; i += nth) to[i] = left.get(i);
+    if (tid == 0) {
+      Q.mode = 0;
+      Q.left = kLeftItems;
+      p.q[qi] = Q;
+      if (alone) {
+        p.ctr->paths = n_paths;
+        p.ctr->res_pin = pin;
+      }
+      p.ctr->stopped = 1;
     }
-    __syncthreads();
-    if (tid == 0) p.q[qi] = Q;
     return;
   }
 
@@ -1673,6 +1724,23 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
   STAMP(7);
 }
 
+// Roots of the queries that outgrew their blocks into the pile the grid launch
+// starts from, after which it may run (one block, a warp per query).
+__global__ void __launch_bounds__(kEngThreads) seed_left_kernel(EngineParams p) {
+  const int pin = p.ctr->res_pin;
+  for (int qi = static_cast<int>(threadIdx.x >> 5); qi < p.nq; qi += kEngWarps) {
+    if (p.q[qi].left != kLeftRoots) continue;
+    seed_query(p, qi, p.q[qi], [&](bool keep, const Item& it) {
+      const unsigned long long slot = warp_append(&p.ctr->pend_out, keep);
+      if (!keep) return;
+      if (slot < p.pend_cap) p.pend[pin][slot] = it;
+      else atomicCAS(&p.ctr->err, kDevOk, kDevCapacity);
+    });
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) p.ctr->restarts = 0;
+}
+
 }  // namespace
 
 int engine_grid(int device, int limit, int* grid_out) {
@@ -1715,6 +1783,11 @@ int launch_engine_blocks(const EngineParams& p, void* stream) {
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   engine_block_kernel<<<p.nq, kEngThreads, smem, static_cast<cudaStream_t>(stream)>>>(p);
+  return cudaGetLastError();
+}
+
+int launch_seed_left(const EngineParams& p, void* stream) {
+  seed_left_kernel<<<1, kEngThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
   return cudaGetLastError();
 }
 

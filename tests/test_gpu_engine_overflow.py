@@ -1,6 +1,6 @@
 """Queries that outgrow what their block of the engine holds: more tied roots
-than frontier slots, path slots reserved past the end of the store, against
-the oracle.  The overflow is detected, nothing behind the end is read, and the
+than frontier slots, path slots reserved past the end of the store, one wall
+of tied paths beside other queries, against the oracle.  The overflow is detected, nothing behind the end is read, and the
 handle answers other queries afterwards."""
 import numpy as np
 import pytest
@@ -15,6 +15,15 @@ def tied_roots(n_src):
     """n_src sources with one unit edge each into one sink: every path costs 1."""
     src = np.arange(n_src, dtype=np.int32)
     return n_src + 1, src, np.full(n_src, n_src, np.int32), np.ones(n_src, np.float32)
+
+
+def tied_wall(diamonds):
+    """2^diamonds paths of the same cost between one source and one sink."""
+    a = 3 * np.arange(diamonds)
+    src = np.stack([a, a, a + 1, a + 2], 1).ravel()
+    dst = np.stack([a + 1, a + 2, a + 3, a + 3], 1).ravel()
+    return (3 * diamonds + 1, src.astype(np.int32), dst.astype(np.int32),
+            np.ones(src.size, np.float32))
 
 
 def generated(seed, n_pins=2000, weight_kind=0):
@@ -82,10 +91,50 @@ def test_tied_roots_of_a_small_query_beside_large_ones():
 
 @pytest.mark.parametrize("queries", [256, 257, 600])
 def test_small_queries_of_the_grid_launch_reserve_past_the_path_store(queries):
-    # a store of 65,536 slots and the graph's source, and 256 slots a query
+    # a store of 65,536 slots and the graph's source, which the chunks that the
+    # blocks take can fill
     graphs = [generated(8)]
     want = expected(graphs[0], 40, 0)
     ks = [1 + q % 40 if queries == 600 else 1 for q in range(queries)]
     got, _ = run_batch(graphs, [0] * queries, ks, cpg_b200.ROOTS_ALL, engine_ctas=8)
     for q in range(queries):
         assert bits_equal(got[q], want[:ks[q]]), q
+
+
+def test_wall_of_ties_beside_others_needs_no_rerun():
+    # 131,072 tied paths for k = 100: more than 300 times its part of the room
+    graphs = [tied_wall(17)] + [generated(20 + i, weight_kind=i % 2) for i in range(3)]
+    gi = [0] + [1 + q % 3 for q in range(47)]
+    ks = [100] + [4000 - q for q in range(47)]
+    got, stats = run_batch(graphs, gi, ks, cpg_b200.ROOTS_REFERENCE)
+    want = [expected(g, 4000, 1) for g in graphs[1:]]
+    assert bits_equal(got[0], np.full(100, 34.0))
+    for q in range(1, 48):
+        assert bits_equal(got[q], want[gi[q] - 1][:ks[q]]), q
+    assert stats["retries"] == 0
+
+
+@pytest.mark.parametrize("beside", [20_000, 4000])
+def test_wall_of_ties_beside_queries_of_the_grid_launch(beside):
+    graphs = [tied_wall(16), generated(30)]
+    got, stats = run_batch(graphs, [0, 1, 0, 1, 1], [7, beside, 300, 50, beside - 1],
+                           cpg_b200.ROOTS_ALL)
+    want = expected(graphs[1], beside, 0)
+    assert bits_equal(got[0], np.full(7, 32.0)) and bits_equal(got[2], np.full(300, 32.0))
+    for q, k in ((1, beside), (3, 50), (4, beside - 1)):
+        assert bits_equal(got[q], want[:k]), q
+
+
+def test_served_wall_of_ties_needs_no_rerun_and_no_allocation():
+    graphs = [tied_wall(17), generated(41), generated(42, weight_kind=1)]
+    want = [None] + [expected(g, 4000, 1) for g in graphs[1:]]
+    with cpg_b200.Server(division=cpg_b200.DIV_IEEE) as s:
+        for g in graphs:
+            s.add_dag(dag_of(g))
+        s.start()
+        asked = [(q % 3, 100 if q % 3 == 0 else 4000 - q) for q in range(60)]
+        for (g, k), t in zip(asked, [s.submit(g, k) for g, k in asked]):
+            costs = s.wait(t)[0]
+            assert bits_equal(costs, np.full(k, 34.0) if g == 0 else want[g][:k]), (g, k)
+        stats = s.stats()
+    assert stats["retries"] == 0 and stats["loop_allocs"] == 0
