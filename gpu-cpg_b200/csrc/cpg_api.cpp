@@ -1083,7 +1083,7 @@ void engine_layout(cpg_handle* h, std::vector<EngineQuery>& qs) {
   };
   unsigned long long all = 0, off = 0, at = 0;
   for (EngineQuery& q : qs) {
-    q.whole = q.k <= whole_max;
+    q.whole = q.k <= whole_max && q.src_end - q.src_beg <= kBlockMaxPend;
     q.out_off = off;
     off += static_cast<unsigned long long>(q.k);
     all += weight(q);
@@ -1107,7 +1107,7 @@ void engine_layout(cpg_handle* h, std::vector<EngineQuery>& qs) {
     }
     if (!whole) {
       h->left_paths = part(h->cap_paths, at);
-      h->left_pend = part(h->cap_pend, at);
+      h->left_pend = qs.size() > 1 ? part(h->cap_pend, at) : h->cap_pend;
     }
   }
 }

@@ -496,6 +496,15 @@ int launch_seed_left(const EngineParams& p, void* stream);
 int launch_engine_blocks(const EngineParams& p, void* stream);
 // Largest k a block answers whole: its sort buffer.
 constexpr long long kBlockMaxK = 16384;
+// More paths or pending items than a block should walk (and 4 k and 8 k): above
+// what k paths take (1.05-1.4 k paths and 3-5 k items, on small graphs up to 3
+// and 10 k), so only ties and many-source graphs get there.  A query that has
+// accepted that many starts again in the grid launch; one with that many
+// pending, if it is alone, leaves it its paths and items.  The lines lie where
+// that is no slower than the block: a wall of 32,768 tied paths (k = 100) takes
+// 0.205 ms on the block against 0.248, one of 131,072 0.647 against 0.279;
+// 20,000 pending sources 0.50 against 0.55, 100,000 2.40 against 2.06.
+constexpr long long kBlockMaxPaths = 49152, kBlockMaxPend = 65536;
 constexpr int kInlineQueries = 8;
 int launch_set_queries(EngineQuery* dst, const EngineQuery* src, int nq, void* stream);
 

@@ -1275,9 +1275,9 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
 // the 20,000-pin graph went from 0.32 to 0.19 ms, the first phases of larger
 // ones by about 0.07 ms.
 //
-// A `whole` query is answered to the end and sorted in shared memory; another
-// one is left to the grid launch at the top of a phase with more than
-// solo_stop items pending.  Blocks never wait on one another, so any number
+// A `whole` query is answered to the end and sorted in shared memory, unless
+// it turns out too large for a block; another one is left to the grid launch at
+// the top of a phase with more than solo_stop items pending.  Blocks never wait on one another, so any number
 // of queries run in one ordinary launch, as many at a time as there are SMs.
 //
 // A block's part of the path store and of the piles is a share.  A query that
@@ -1287,6 +1287,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_kernel(EngineParams p) {
 // queries together, not on a share.
 constexpr unsigned kBlkPend = 4096, kBlkFront = 1536;
 constexpr int kChunks = 64;  // path chunks of a query that leaves its paths
+constexpr int kGoOutgrown = 2;
 
 struct BlockMem {
   Item pend[2][kBlkPend];
@@ -1406,6 +1407,8 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
     s_pend[0] = s_pend[1] = 0;
     s_chunk[0] = s_chunk[1] = 0;
     s_chunks = 0;
+    if (!Q.whole && p.nq > 1) Q.path_cap = ~0ull;  // (its slots come in chunks)
+    Q.path_cap = min(Q.path_cap, max(kBlockMaxPaths, 4 * min(Q.k, kBlockMaxK)));
   }
   for (int i = tid; i < kSelBins; i += nth) m.hist[i] = 0;  // every pick leaves it zero again
   __syncthreads();
@@ -1442,15 +1445,19 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
     if (tid == 0) {
       // (paths in chunks: the final phase, which selects over them, is the
       // grid's)
-      const bool stay = whole || (n_pend <= p.solo_stop &&
-                                  (alone || Q.paths_nz < static_cast<unsigned long long>(Q.k)));
-      s_go = stay && decide_query(p, Q);
+      const unsigned long long most = whole ? max(kBlockMaxPend, 8 * Q.k) : p.solo_stop;
+      const bool stay = Q.done || (n_pend <= most &&
+                                   (own || Q.paths_nz < static_cast<unsigned long long>(Q.k)));
+      s_go = !stay ? (whole && !alone ? kGoOutgrown : 0) : decide_query(p, Q);
       s_pend[pin ^ 1] = 0;
       s_front[0] = s_front[1] = s_front[2] = 0;
       s_nz = s_pnz = 0;
     }
     __syncthreads();
-    if (!s_go) break;
+    if (s_go != 1) {
+      outgrown = s_go == kGoOutgrown;
+      break;
+    }
     STAMP(1);
     const BlkPile pile = pend_pile(pin), next = pend_pile(pin ^ 1);
     // select
@@ -1519,7 +1526,8 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
       }
       const unsigned long long base = own ? Q.path_base + n_paths : s_base;
       // (the same for every thread)
-      if (own ? n_paths + n > Q.path_cap : base + n > p.left_paths || s_chunks == kChunks) {
+      if (n_paths + n > Q.path_cap ||
+          (!own && (base + n > p.left_paths || s_chunks == kChunks))) {
         outgrown = true;
         break;
       }
@@ -1570,11 +1578,12 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
   }
 
   const unsigned n_pend = s_pend[pin];
+  const bool leaves = !whole || !Q.done;
   if (tid == 0) {
     atomicMax(&p.ctr->res_phase, phase);
     atomicMax(&p.ctr->phases, phase);
     atomicAdd(&p.ctr->rounds, rounds);
-    if (!whole && !outgrown) {
+    if (leaves && !outgrown) {
       // room for the pending items in the pile the grid launch starts from
       unsigned long long at = 0, seen;
       do {
@@ -1586,7 +1595,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
     }
   }
   __syncthreads();
-  if (!whole && !outgrown) outgrown = !s_fits;
+  if (leaves && !outgrown) outgrown = !s_fits;
   if (!own) {
     // slots without a path; the paths of a query that starts again are no part
     // of the answer
@@ -1608,7 +1617,7 @@ __global__ void __launch_bounds__(kEngThreads) engine_block_kernel(EngineParams 
     }
     return;
   }
-  if (!whole) {
+  if (leaves) {
     // the rest is the grid's, which decides the next phase.  (A query alone
     // spilled into the very pile: its other items join behind those.)
     const unsigned spilled = alone && n_pend > kBlkPend ? n_pend - kBlkPend : 0;

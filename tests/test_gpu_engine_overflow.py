@@ -138,3 +138,32 @@ def test_served_wall_of_ties_needs_no_rerun_and_no_allocation():
             assert bits_equal(costs, np.full(k, 34.0) if g == 0 else want[g][:k]), (g, k)
         stats = s.stats()
     assert stats["retries"] == 0 and stats["loop_allocs"] == 0
+
+
+@pytest.mark.parametrize("k", [1, 100, 4096, 5000])
+@pytest.mark.parametrize("diamonds", [15, 16, 18])
+def test_tied_paths_around_what_a_block_walks(diamonds, k):
+    with cpg_b200.CpGen(division=cpg_b200.DIV_IEEE) as g:
+        g.load_edges(*tied_wall(diamonds))
+        g.report_paths(k)
+        nodes = g.get_pfxt_nodes(k)
+        assert bits_equal(g.get_slacks(k), np.full(k, 2.0 * diamonds))
+        assert bits_equal(nodes["slack"], np.full(k, 2.0 * diamonds))
+        v = g.path_vertices(k - 1)
+        assert v[0] == 0 and v[-1] == 3 * diamonds and v.size == 2 * diamonds + 1
+
+
+@pytest.mark.parametrize("n_src", [4097, 65536, 65537, 90_000])
+@pytest.mark.parametrize("k", [50, 4096])
+def test_many_sources_alone_and_beside_others(n_src, k):
+    w = np.random.default_rng(n_src).uniform(1, 100, n_src).astype(np.float32)
+    graphs = [tied_roots(n_src)[:3] + (w,), generated(31)]
+    want = [expected(graphs[0], k, 0), expected(graphs[1], 700, 0)]
+    with cpg_b200.CpGen(division=cpg_b200.DIV_IEEE, root_seeding=cpg_b200.ROOTS_ALL) as g:
+        g.load_edges(*graphs[0])
+        g.report_paths(k)
+        assert bits_equal(g.get_slacks(k), want[0])
+        assert g.path_vertices(0).size == 2
+    got, _ = run_batch(graphs, [1, 0, 1], [700, k, 20], cpg_b200.ROOTS_ALL)
+    assert bits_equal(got[0], want[1]) and bits_equal(got[1], want[0])
+    assert bits_equal(got[2], want[1][:20])
