@@ -39,13 +39,23 @@ constexpr unsigned int kDefaultSpinLimit = 1u << 24;
 constexpr size_t kPinnedBytes = 4096;
 // pending items up to which a query's block runs its phases
 constexpr unsigned long long kEngSoloStop = 4096;
-// k up to which a block answers a query to the end.  Alone on the device it
-// is ahead of the grid launch up to about 4,000 (1M-pin graph: 0.147 against
-// 0.212 ms at k = 1,000, 0.322 against 0.347 at 4,000; one CTA of the grid
-// launch takes 0.64 against 0.36 ms at 8,000).  Beside other queries, which
-// keep the other SMs busy, up to what its sort buffer holds: 48 served
-// requests of k up to 20,000 take 6.3 ms, against 9.8 ms in grid launches.
-constexpr long long kWholeAlone = 4096, kWholeBeside = kBlockMaxK;
+// k up to which a block answers a query to the end, where that is no slower
+// than the grid launch.
+//
+// Alone: the block is ahead up to about 4,300 on graphs of mean degree 2.5 and
+// 5 (20,000 to 400,000 pins, fp32 and integer delays: 0.21 against 0.27 ms at
+// k = 2,000, 0.28 against 0.29 at 4,000, 0.34 against 0.30 at 5,000), up to
+// 3,000 at mean degree 10 and 2,500 at 20 (1M pins: 0.240 against 0.271 ms at
+// 2,000, 0.316 against 0.302 at 3,000), where a path brings more items.
+//
+// Beside others the grid launch costs more and the blocks share nothing: two
+// queries cross at 11,000 (mean degree 20; 0.45 against 0.57 ms at 8,000, 0.71
+// against 0.61 at 16,000), four at 12,500, eight at what the block's sort
+// holds; 48 of k = 16,000 take 0.77 against 1.52 ms.
+long long whole_limit(const HostGraph& g, size_t nq) {
+  if (nq > 1) return std::min<long long>(kBlockMaxK, 8192 + 1024 * static_cast<long long>(nq));
+  return g.m < int64_t{8} * g.n ? 4096 : 2560;
+}
 enum { kRetry = 1000 };  // internal: a bounded buffer overflowed, grow and rerun
 constexpr int32_t kMaxRow = 16384;  // longest deviation row the row sort takes
 
@@ -1076,7 +1086,7 @@ int try_query(cpg_handle* h, unsigned long long k) {
 // growth phases overshoot k by more: among 48 of k up to 50,000 one of
 // k = 2,554 had 25,400 items pending and outgrew 8 k and the block's own 4,096.
 void engine_layout(cpg_handle* h, std::vector<EngineQuery>& qs) {
-  const long long whole_max = h->opts.engine_ctas > 0 ? 0 : qs.size() > 1 ? kWholeBeside : kWholeAlone;
+  const long long whole_max = h->opts.engine_ctas > 0 ? 0 : whole_limit(h->g, qs.size());
   auto weight = [](const EngineQuery& q) {
     return static_cast<unsigned long long>(std::min<long long>(q.k, kBlockMaxK)) + 2048 +
            static_cast<unsigned long long>(q.src_end - q.src_beg);

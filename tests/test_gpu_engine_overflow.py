@@ -167,3 +167,27 @@ def test_many_sources_alone_and_beside_others(n_src, k):
     got, _ = run_batch(graphs, [1, 0, 1], [700, k, 20], cpg_b200.ROOTS_ALL)
     assert bits_equal(got[0], want[1]) and bits_equal(got[1], want[0])
     assert bits_equal(got[2], want[1][:20])
+
+
+@pytest.mark.parametrize("k", [2559, 2560, 2561])
+def test_dense_graph_around_the_whole_limit(k):
+    d = cpg_b200.generate(cpg_b200.gen_params(
+        seed=3, n_pins=1500, n_levels=12, n_first=8, n_last=8, level_span=3, degree_kind=1,
+        deg_mean=12.0, deg_cap=40, add_virtual=1))
+    assert d.m >= 8 * d.n
+    graph = (d.n, d.src, d.dst, d.w)
+    with cpg_b200.CpGen(division=cpg_b200.DIV_IEEE) as g:
+        g.load_edges(*graph)
+        g.report_paths(k)
+        assert bits_equal(g.get_slacks(k), expected(graph, k, 1))
+
+
+@pytest.mark.parametrize("queries", [2, 5, 8])
+def test_few_queries_around_the_whole_limit(queries):
+    graphs = [generated(50 + i, weight_kind=i % 2) for i in range(2)]
+    line = min(16384, 8192 + 1024 * queries)
+    ks = [line - 1 + q % 3 for q in range(queries)]
+    want = [expected(g, line + 1, 0) for g in graphs]
+    got, _ = run_batch(graphs, [q % 2 for q in range(queries)], ks, cpg_b200.ROOTS_ALL)
+    for q in range(queries):
+        assert bits_equal(got[q], want[q % 2][:ks[q]]), q
