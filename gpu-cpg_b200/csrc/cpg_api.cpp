@@ -48,13 +48,17 @@ constexpr unsigned long long kEngSoloStop = 4096;
 // 3,000 at mean degree 10 and 2,500 at 20 (1M pins: 0.240 against 0.271 ms at
 // 2,000, 0.316 against 0.302 at 3,000), where a path brings more items.
 //
-// Beside others the grid launch costs more and the blocks share nothing: two
-// queries cross at 11,000 (mean degree 20; 0.45 against 0.57 ms at 8,000, 0.71
-// against 0.61 at 16,000), four at 12,500, eight at what the block's sort
-// holds; 48 of k = 16,000 take 0.77 against 1.52 ms.
-long long whole_limit(const HostGraph& g, size_t nq) {
-  if (nq > 1) return std::min<long long>(kBlockMaxK, 8192 + 1024 * static_cast<long long>(nq));
-  return g.m < int64_t{8} * g.n ? 4096 : 2560;
+// Beside others: what the block's sort holds, since the grid launch costs more
+// for several queries and comes behind the blocks of the small ones (48 of
+// k = 16,000 take 0.77 against 1.52 ms), unless every query is large and they
+// are few: two cross at 11,000 (mean degree 20; 0.45 against 0.57 ms at 8,000,
+// 0.71 against 0.61 at 16,000), four at 12,500, eight at 16,000.
+long long whole_limit(const HostGraph& g, const std::vector<EngineQuery>& qs) {
+  if (qs.size() == 1) return g.m < int64_t{8} * g.n ? 4096 : 2560;
+  const long long few = 8192 + 1024 * static_cast<long long>(qs.size());
+  for (const EngineQuery& q : qs)
+    if (q.k <= few) return kBlockMaxK;
+  return std::min<long long>(kBlockMaxK, few);
 }
 enum { kRetry = 1000 };  // internal: a bounded buffer overflowed, grow and rerun
 constexpr int32_t kMaxRow = 16384;  // longest deviation row the row sort takes
@@ -1086,7 +1090,7 @@ int try_query(cpg_handle* h, unsigned long long k) {
 // growth phases overshoot k by more: among 48 of k up to 50,000 one of
 // k = 2,554 had 25,400 items pending and outgrew 8 k and the block's own 4,096.
 void engine_layout(cpg_handle* h, std::vector<EngineQuery>& qs) {
-  const long long whole_max = h->opts.engine_ctas > 0 ? 0 : whole_limit(h->g, qs.size());
+  const long long whole_max = h->opts.engine_ctas > 0 ? 0 : whole_limit(h->g, qs);
   auto weight = [](const EngineQuery& q) {
     return static_cast<unsigned long long>(std::min<long long>(q.k, kBlockMaxK)) + 2048 +
            static_cast<unsigned long long>(q.src_end - q.src_beg);

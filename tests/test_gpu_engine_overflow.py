@@ -186,8 +186,9 @@ def test_dense_graph_around_the_whole_limit(k):
 def test_few_queries_around_the_whole_limit(queries):
     graphs = [generated(50 + i, weight_kind=i % 2) for i in range(2)]
     line = min(16384, 8192 + 1024 * queries)
-    ks = [line - 1 + q % 3 for q in range(queries)]
-    want = [expected(g, line + 1, 0) for g in graphs]
-    got, _ = run_batch(graphs, [q % 2 for q in range(queries)], ks, cpg_b200.ROOTS_ALL)
-    for q in range(queries):
-        assert bits_equal(got[q], want[q % 2][:ks[q]]), q
+    want = [expected(g, line + 3, 0) for g in graphs]
+    for least in (line - 1, line, line + 1):
+        ks = [least + q % 3 for q in range(queries)]
+        got, _ = run_batch(graphs, [q % 2 for q in range(queries)], ks, cpg_b200.ROOTS_ALL)
+        for q in range(queries):
+            assert bits_equal(got[q], want[q % 2][:ks[q]]), q
