@@ -115,6 +115,7 @@ struct cpg_handle {
   DevMem d_order, d_lvlp, d_level_of, d_dist, d_succ, d_dev_cnt, d_dev,
       d_ht_root, d_ht_size, d_hnodes, d_pool_mark, d_deps, d_sctr, d_best;
   unsigned long long hnode_cap = 0;
+  unsigned long long hnode_extra = 0;  // nodes a vertex on top of what a build needs (served form)
 
   // query
   unsigned long long cap_paths = 0, cap_front = 0, cap_pend = 0;
@@ -401,9 +402,19 @@ Status upload_graph(cpg_handle* h, int32_t n, int32_t m, const int32_t* adjp,
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
   const unsigned long long want = nn * 10ull + 1024 + 64ull * 32 * static_cast<unsigned>(sms);
-  if (h->hnode_cap < want) {
-    h->hnode_cap = want;
+  const unsigned long long most = want + nn * h->hnode_extra;
+  if (h->hnode_cap < most) {
     release(h->d_hnodes);
+    // the extra room only if the device has it to spare
+    size_t free_b = 0, total_b = 0;
+    const bool spare = most > want && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+                       most * sizeof(HeapNode) < free_b / 4;
+    if (spare && ensure(h->d_hnodes, most * sizeof(HeapNode)) == cudaSuccess) {
+      h->hnode_cap = most;
+    } else {
+      cudaGetLastError();
+      h->hnode_cap = std::max(h->hnode_cap, want);
+    }
   }
   CK(ensure(h->d_hnodes, h->hnode_cap * sizeof(HeapNode)), "alloc chain heaps");
   cudaStream_t s = h->stream;
@@ -2610,28 +2621,12 @@ cpg_status cpg_server_add_dag(cpg_server* sv, const cpg_dag* d, int32_t* graph_i
 
 cpg_status cpg_server_start(cpg_server* sv) {
   if (!sv || sv->running) return CPG_ERR_INVALID;
+  // Rebuilds after delay updates append their chain heaps to the pool, and one
+  // that overflows it is done again for every graph: room for two more trees (a
+  // tree takes about 7 nodes a vertex, the pool has 10).
+  sv->b->h->hnode_extra = 14;
   cpg_status st = cpg_batch_commit(sv->b);
   if (st != CPG_OK) return st;
-  {
-    // Rebuilds after delay updates append their chain heaps to the pool, and
-    // one that overflows it is done again for every graph: room for two more
-    // trees (a tree takes about 7 nodes a vertex, the pool has 10), if the
-    // device has it to spare.
-    cpg_handle* h = sv->b->h;
-    const unsigned long long want = h->hnode_cap + 14ull * static_cast<unsigned long long>(h->g.n);
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && want * sizeof(HeapNode) < free_b / 4) {
-      const unsigned long long had = h->hnode_cap;
-      release(h->d_hnodes);
-      h->hnode_cap = want;
-      if (ensure(h->d_hnodes, want * sizeof(HeapNode)) != cudaSuccess) {
-        cudaGetLastError();
-        h->hnode_cap = had;
-        const Status ws = ensure(h->d_hnodes, had * sizeof(HeapNode)) == cudaSuccess ? CPG_OK : CPG_ERR_OOM;
-        if (ws != CPG_OK) return fail(h, ws, "alloc chain heaps");
-      }
-    }
-  }
   st = cpg_levelize(sv->b->h);
   if (st != CPG_OK) return st;
   // The engine's path and item piles, sized once for a launch answering

@@ -120,3 +120,25 @@ def test_server_many_updates_rebuild_only_changed_graphs():
             h.report_paths(k)
             alone = h.get_slacks(k)
         assert np.array_equal(mixed[i].view(np.uint32), alone.view(np.uint32)), i
+
+
+def test_start_stop_start_answers_alike_and_keeps_its_memory():
+    import torch
+    dags = [cpg_b200.generate(cpg_b200.gen_params(seed=60 + i, n_pins=50_000, n_levels=60, n_first=32,
+                                                  n_last=32, level_span=3)) for i in range(4)]
+    qs = _stream(dags, 24, seed=9)
+    free, first = [], None
+    with cpg_b200.Server(max_batch=16) as s:
+        for d in dags:
+            s.add_dag(d)
+        for _ in range(4):
+            s.start()
+            free.append(torch.cuda.mem_get_info()[0])
+            tickets = [s.submit(g, k, *(upd if upd else (None, None))) for g, k, upd in qs]
+            out = [s.wait(t, timeout_ms=120000)[0] for t in tickets]
+            s.stop()
+            if first is None:
+                first = out
+            assert all(np.array_equal(a.view(np.uint32), b.view(np.uint32)) for a, b in zip(out, first))
+    # a start that enlarged the heap pool again would take 90 MB more each time
+    assert free[1] - free[3] < 32 << 20 and free[0] - free[1] < 64 << 20
