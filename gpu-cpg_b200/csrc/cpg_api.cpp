@@ -680,6 +680,7 @@ SfxtParams sfxt_params(cpg_handle* h, int32_t start_level, bool known = false) {
 Status enqueue_sfxt(cpg_handle* h, int32_t start_level, int* launches,
                     bool kernel_events = false, bool known = false) {
   cudaStream_t s = h->stream;
+  if (!h->d_hnodes.p) CK(ensure(h->d_hnodes, pool_bytes(h->hnode_cap, h->g.n)), "alloc chain heaps");
   if (h->multi_graph && start_level > 0) {
     CK(cudaMemcpyAsync(h->d_graph_from.p, h->graph_from.data(), h->graph_from.size() * 4,
                        cudaMemcpyHostToDevice, s), "H2D changed levels");
@@ -734,10 +735,17 @@ int finish_sfxt(cpg_handle* h, int32_t start_level, bool known = false) {
 }
 
 Status grow_heap_pool(cpg_handle* h) {
+  h->sfxt_valid = false;  // the pool's contents go
   release(h->d_hnodes);
-  h->hnode_cap *= 2;
-  CK(ensure(h->d_hnodes, pool_bytes(h->hnode_cap, h->g.n)), "alloc chain heaps");
-  return CPG_OK;
+  const cudaError_t e = ensure(h->d_hnodes, pool_bytes(2 * h->hnode_cap, h->g.n));
+  if (e == cudaSuccess) {
+    h->hnode_cap *= 2;
+    return CPG_OK;
+  }
+  // the old size again, so that a later build finds a pool (enqueue_sfxt looks)
+  cudaGetLastError();
+  if (ensure(h->d_hnodes, pool_bytes(h->hnode_cap, h->g.n)) != cudaSuccess) cudaGetLastError();
+  return cuda_fail(h, e, "alloc chain heaps");
 }
 
 Status run_sfxt(cpg_handle* h, int32_t start_level, bool known = false) {
@@ -2047,9 +2055,9 @@ int batch_step(cpg_batch* b, bool rebuild) {
   if (rebuild) {
     const int r = finish_sfxt(h, 0);
     if (r == kRetry) {
+      batch_drop_graph(b);  // it names the old pool
       Status st = grow_heap_pool(h);
       if (st != CPG_OK) return st;
-      batch_drop_graph(b);
       return kRetry;
     }
     if (r != CPG_OK) return r;
