@@ -2532,15 +2532,23 @@ void server_loop(cpg_server* sv) {
     }
     const double t_sfxt = now_s();
     std::vector<std::vector<float>> out;
-    for (int attempt = 0; st == CPG_OK && attempt < 10; ++attempt) {
-      const int r = server_launch(sv, batch, out);
+    const unsigned long long caps[3] = {h->cap_paths, h->cap_front, h->cap_pend};
+    int r = st == CPG_OK ? static_cast<int>(kRetry) : static_cast<int>(st);
+    for (int attempt = 0; r == kRetry && attempt < 10; ++attempt) {
+      r = server_launch(sv, batch, out);
       if (r == kRetry) {
         grow_caps(h);
         sv->retries += 1;
-        continue;
       }
-      st = static_cast<Status>(r);
-      break;
+    }
+    if (r == kRetry) r = fail(h, CPG_ERR_CAPACITY, "engine buffers cannot grow further");
+    st = static_cast<Status>(r);
+    if (st != CPG_OK) {
+      // a launch that asked for more than there is must not leave its
+      // capacities to the launches behind it
+      h->cap_paths = caps[0];
+      h->cap_front = caps[1];
+      h->cap_pend = caps[2];
     }
     const double t = now_s();
     {

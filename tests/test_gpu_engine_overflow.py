@@ -192,3 +192,22 @@ def test_few_queries_around_the_whole_limit(queries):
         got, _ = run_batch(graphs, [q % 2 for q in range(queries)], ks, cpg_b200.ROOTS_ALL)
         for q in range(queries):
             assert bits_equal(got[q], want[q % 2][:ks[q]]), q
+
+
+def test_served_query_that_needs_more_than_there_is_fails_alone():
+    graphs = [tied_wall(20), generated(45)]
+    want = expected(graphs[1], 2000, 1)
+    try:
+        with cpg_b200.Server(division=cpg_b200.DIV_IEEE, hbm_budget_bytes=64 << 20) as s:
+            for g in graphs:
+                s.add_dag(dag_of(g))
+            s.start()
+            cpg_b200.debug_fail_allocs_above(4 << 20)   # a million tied paths need more
+            with pytest.raises(cpg_b200.CpgError) as e:
+                s.wait(s.submit(0, 100))
+            assert e.value.status == 3                  # out of memory
+            assert bits_equal(s.wait(s.submit(1, 2000))[0], want)
+            cpg_b200.debug_fail_allocs_above(0)
+            assert bits_equal(s.wait(s.submit(0, 100))[0], np.full(100, 40.0))
+    finally:
+        cpg_b200.debug_fail_allocs_above(0)
