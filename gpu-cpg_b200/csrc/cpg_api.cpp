@@ -1605,36 +1605,54 @@ cpg_status cpg_update_delays(cpg_handle* h, int64_t count, const int32_t* eids,
     }
     eids = mapped.data();
   }
-  // The device checks the ids and finds the changed tails' lowest level per
-  // graph, then writes the delays.  Staging kept by the handle: no allocation
-  // (and no device-wide synchronisation) per update.
   const bool have_levels = h->sfxt_valid || h->dirty_level > 0;
   const size_t ng = h->multi_graph ? h->graph_from.size() : 1;
-  CK(ensure_grow(h->d_upd, static_cast<size_t>(count) * 8), "alloc delay update");
-  CK(ensure_grow(h->d_located, (ng + 1) * 4), "alloc delay update");
-  int32_t* up_e = P<int32_t>(h->d_upd);
-  float* up_w = reinterpret_cast<float*>(up_e + count);
-  CK(cudaMemcpyAsync(up_e, eids, count * 4, cudaMemcpyHostToDevice, h->stream), "H2D eids");
-  CK(cudaMemcpyAsync(up_w, w, count * 4, cudaMemcpyHostToDevice, h->stream), "H2D delays");
   SfxtParams up = sfxt_params(h, 0);
   up.vgraph = h->multi_graph ? P<int32_t>(h->d_vgraph) : nullptr;
-  CK(launch_update_delays(up, P<DevEdge>(h->d_edges), h->g.m, up_e, up_w, count, have_levels,
-                          P<int32_t>(h->d_located), static_cast<int32_t>(ng), h->stream),
-     "delay update");
   std::vector<int32_t> far;  // more graphs than the pinned staging holds
   int32_t* located = static_cast<int32_t*>(h->pinned);
-  if ((ng + 1) * 4 > kPinnedBytes) {
-    far.resize(ng + 1);
-    located = far.data();
+  static_assert((3 * kFewUpdates + kFewGraphs) * 4 <= kPinnedBytes, "pinned staging");
+  if (count <= kFewUpdates && ng <= static_cast<size_t>(kFewGraphs)) {
+    int32_t* in = located + kFewGraphs;
+    const int few = static_cast<int>(count);
+    for (int i = 0; i < few; ++i) {
+      const int32_t e = eids[i];
+      if (e < 0 || e >= h->g.m) return fail(h, CPG_ERR_INVALID, "edge id out of range");
+      in[i] = e;
+      in[few + i] = static_cast<int32_t>(
+          std::upper_bound(h->g.adjp.begin(), h->g.adjp.end(), e) - h->g.adjp.begin() - 1);
+    }
+    std::memcpy(in + 2 * few, w, static_cast<size_t>(few) * 4);
+    CK(launch_update_few(up, P<DevEdge>(h->d_edges), in, few, have_levels, located,
+                         static_cast<int32_t>(ng), h->stream),
+       "delay update");
+    CK(cudaStreamSynchronize(h->stream), "delay update");
+  } else {
+    // The device checks the ids and finds the changed tails' lowest level per
+    // graph, then writes the delays.  Staging kept by the handle: no allocation
+    // (and no device-wide synchronisation) per update.
+    CK(ensure_grow(h->d_upd, static_cast<size_t>(count) * 8), "alloc delay update");
+    CK(ensure_grow(h->d_located, (ng + 1) * 4), "alloc delay update");
+    int32_t* up_e = P<int32_t>(h->d_upd);
+    float* up_w = reinterpret_cast<float*>(up_e + count);
+    CK(cudaMemcpyAsync(up_e, eids, count * 4, cudaMemcpyHostToDevice, h->stream), "H2D eids");
+    CK(cudaMemcpyAsync(up_w, w, count * 4, cudaMemcpyHostToDevice, h->stream), "H2D delays");
+    CK(launch_update_delays(up, P<DevEdge>(h->d_edges), h->g.m, up_e, up_w, count, have_levels,
+                            P<int32_t>(h->d_located), static_cast<int32_t>(ng), h->stream),
+       "delay update");
+    if ((ng + 1) * 4 > kPinnedBytes) {
+      far.resize(ng + 1);
+      located = far.data();
+    }
+    CK(cudaMemcpyAsync(located, h->d_located.p, (ng + 1) * 4, cudaMemcpyDeviceToHost, h->stream),
+       "D2H changed levels");
+    CK(cudaStreamSynchronize(h->stream), "delay update");
+    if (*located++ != 0) return fail(h, CPG_ERR_INVALID, "edge id out of range");
   }
-  CK(cudaMemcpyAsync(located, h->d_located.p, (ng + 1) * 4, cudaMemcpyDeviceToHost, h->stream),
-     "D2H changed levels");
-  CK(cudaStreamSynchronize(h->stream), "delay update");
-  if (located[0] != 0) return fail(h, CPG_ERR_INVALID, "edge id out of range");
   int32_t lowest = INT32_MAX;
   for (size_t g = 0; g < ng; ++g) {
-    lowest = std::min(lowest, located[1 + g]);
-    if (h->multi_graph) h->graph_from[g] = std::min(h->graph_from[g], located[1 + g]);
+    lowest = std::min(lowest, located[g]);
+    if (h->multi_graph) h->graph_from[g] = std::min(h->graph_from[g], located[g]);
   }
   // incremental rebuild from the lowest changed level (levels never change
   // with delays); without levels a full rebuild follows

@@ -556,6 +556,13 @@ int launch_topk_costs(const float* costs, unsigned long long n, unsigned long lo
                       const TopkScratch& s, float* out, unsigned long long* n_out,
                       void* stream);
 
+// Up to kFewUpdates new delays, checked by the host: in (pinned) holds their
+// edge ids, tails and delays, out (pinned) receives the lowest changed level of
+// each of up to kFewGraphs graphs.
+constexpr int kFewUpdates = 256, kFewGraphs = 128;
+int launch_update_few(const SfxtParams& p, DevEdge* edges, const int32_t* in, int count,
+                      bool have_levels, int32_t* out, int32_t ng, void* stream);
+
 // Checks, locates (lowest changed level per graph) and writes new delays.
 int launch_update_delays(const SfxtParams& p, DevEdge* edges, int32_t m, const int32_t* eids,
                          const float* w, int64_t count, bool have_levels, int32_t* out,

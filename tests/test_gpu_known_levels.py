@@ -152,3 +152,53 @@ def test_rows_at_the_edges_of_the_register_words(deg, heap_mode):
             e = rng.choice(adj.size, 1 + adj.size // 3, replace=False).astype(np.int32)
             w[e] = rng.integers(1, 6, e.size).astype(np.float32)
             g.update_delays(e, w[e])
+
+
+@pytest.mark.parametrize("count", [1, 2, 255, 256, 257, 300])
+def test_few_updates_one_by_one_equal_a_fresh_upload(count):
+    n, src, dst, w = cases.load_case("small_f32_s12")
+    adjp, adj, w = _csr(n, src, dst, w)
+    rng = np.random.default_rng(count)
+    with cpg_b200.CpGen(division=cpg_b200.DIV_IEEE) as g, cpg_b200.CpGen(division=cpg_b200.DIV_IEEE) as f:
+        g.load_csr(n, adjp, adj, w)
+        for step in range(3):   # before any levels, with a current tree, and twice in a row
+            e = rng.choice(w.size, count, replace=False).astype(np.int32)
+            w[e] = rng.uniform(0.1, 10, count).astype(np.float32)
+            g.update_delays(e, w[e])
+            for bad in (-1, w.size):
+                with pytest.raises(cpg_b200.CpgError) as err:
+                    g.update_delays(np.r_[e[:-1], bad].astype(np.int32), np.zeros(count, np.float32))
+                assert err.value.status == 1
+            if step != 1:
+                g.report_paths(1500)
+        f.load_csr(n, adjp, adj, w)
+        f.report_paths(1500)
+        assert np.array_equal(g.get_slacks(1500).view(np.uint32), f.get_slacks(1500).view(np.uint32))
+        for a, b in zip(g.get_sfxt(), f.get_sfxt()):
+            np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("graphs", [1, 127, 128, 129])
+def test_few_updates_of_many_side_by_side_graphs(graphs):
+    d = cpg_b200.generate(cpg_b200.gen_params(seed=5, n_pins=60, n_levels=5, n_first=3, n_last=3,
+                                              level_span=2, degree_kind=0, deg_lo=1, deg_hi=3))
+    adjp, adj, w = _csr(d.n, d.src, d.dst, d.w)
+    e = np.arange(0, w.size, 3, dtype=np.int32)
+    x = np.linspace(0.5, 9.5, e.size).astype(np.float32)
+    changed = w.copy()
+    changed[e] = x
+    want = []
+    for v in (w, changed):
+        og = oracle.OracleGraph.from_edges(d.n, np.repeat(np.arange(d.n, dtype=np.int32), np.diff(adjp)), adj, v)
+        want.append(og.closure_topk(30)[0]["slack"].astype(np.float32))
+    with cpg_b200.Server(division=cpg_b200.DIV_IEEE) as s:
+        for _ in range(graphs):
+            s.add_graph(d.n, adjp, adj, w)
+        s.start()
+        hit = {0, graphs // 2, graphs - 1}
+        for g in hit:
+            got = s.wait(s.submit(g, 30, e, x))[0]
+            assert np.array_equal(got.view(np.uint32), want[1].view(np.uint32)), g
+        for g in range(0, graphs, 7):
+            got = s.wait(s.submit(g, 30))[0]
+            assert np.array_equal(got.view(np.uint32), want[g in hit].view(np.uint32)), g
