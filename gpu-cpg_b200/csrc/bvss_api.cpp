@@ -38,6 +38,10 @@ struct cpg_bvss {
   std::string err;
   int device = -1;  // device holding the copy below
   Buf d_ptr, d_v2r, d_cnt, d_rows, d_masks, d_scratch, d_ctr, d_io, d_out;
+  // around the device work of a run, and where its counters come back (a call
+  // of few sources is bound by what it does besides the kernels)
+  cudaEvent_t ev[2] = {};
+  BvssCounters* counters = nullptr;  // pinned
 };
 
 namespace {
@@ -57,6 +61,22 @@ Status bfail(cpg_bvss* b, Status s, const std::string& msg) {
     }                                                                          \
   } while (0)
 
+void drop_device(cpg_bvss* b) {
+  Buf* all[] = {&b->d_ptr, &b->d_v2r, &b->d_cnt, &b->d_rows, &b->d_masks,
+                &b->d_scratch, &b->d_ctr, &b->d_io, &b->d_out};
+  for (Buf* x : all) {
+    if (x->p) cudaFree(x->p);
+    *x = Buf{};
+  }
+  for (cudaEvent_t& x : b->ev) {
+    if (x) cudaEventDestroy(x);
+    x = nullptr;
+  }
+  if (b->counters) cudaFreeHost(b->counters);
+  b->counters = nullptr;
+  b->device = -1;
+}
+
 Status upload(cpg_bvss* b, int device) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
@@ -66,12 +86,9 @@ Status upload(cpg_bvss* b, int device) {
   if (device < 0 || device >= ndev) return bfail(b, CPG_ERR_INVALID, "bad device ordinal");
   BCK(cudaSetDevice(device), "cudaSetDevice");
   if (b->device == device) return CPG_OK;
-  Buf* all[] = {&b->d_ptr, &b->d_v2r, &b->d_cnt, &b->d_rows, &b->d_masks,
-                &b->d_scratch, &b->d_ctr, &b->d_io, &b->d_out};
-  for (Buf* x : all) {
-    if (x->p) cudaFree(x->p);
-    *x = Buf{};
-  }
+  drop_device(b);
+  for (cudaEvent_t& x : b->ev) BCK(cudaEventCreate(&x), "event");
+  BCK(cudaMallocHost(&b->counters, sizeof(BvssCounters)), "alloc BVSS");
   const HostBvss& h = b->hb;
   BCK(grow(b->d_ptr, h.ptr.size() * 4), "alloc BVSS");
   BCK(grow(b->d_v2r, h.v2r.size() * 4), "alloc BVSS");
@@ -194,13 +211,8 @@ cpg_status cpg_bvss_build_compact(cpg_bvss** out, int32_t n, const int32_t* devi
 
 void cpg_bvss_destroy(cpg_bvss* b) {
   if (!b) return;
-  if (b->device >= 0) {
-    cudaSetDevice(b->device);
-    Buf* all[] = {&b->d_ptr, &b->d_v2r, &b->d_cnt, &b->d_rows, &b->d_masks,
-                  &b->d_scratch, &b->d_ctr, &b->d_io, &b->d_out};
-    for (Buf* x : all)
-      if (x->p) cudaFree(x->p);
-  }
+  if (b->device >= 0) cudaSetDevice(b->device);
+  drop_device(b);
   delete b;
 }
 
@@ -308,9 +320,7 @@ cpg_status cpg_bvss_levels(cpg_bvss* b, const cpg_bvss_opts* opts, const int32_t
   BCK(grow(b->d_io, static_cast<size_t>(n_sinks) * 4), "alloc BVSS sinks");
   BCK(grow(b->d_out, static_cast<size_t>(h.n_rows) * 4), "alloc BVSS levels");
   cudaStream_t s = static_cast<cudaStream_t>(o.stream);
-  cudaEvent_t e0, e1;
-  BCK(cudaEventCreate(&e0), "event");
-  BCK(cudaEventCreate(&e1), "event");
+  const cudaEvent_t e0 = b->ev[0], e1 = b->ev[1];
   cudaError_t e = cudaSuccess;
   if (n_sinks) e = cudaMemcpyAsync(b->d_io.p, sinks, static_cast<size_t>(n_sinks) * 4,
                                    cudaMemcpyHostToDevice, s);
@@ -322,7 +332,7 @@ cpg_status cpg_bvss_levels(cpg_bvss* b, const cpg_bvss_opts* opts, const int32_t
         static_cast<BvssCounters*>(b->d_ctr.p), dispatch(o),
         o.spin_limit ? o.spin_limit : kBvssSpinLimit, o.device, s));
   if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-  BvssCounters c{};
+  BvssCounters& c = *b->counters;
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&c, b->d_ctr.p, sizeof(c), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && h.n_rows)
@@ -331,8 +341,6 @@ cpg_status cpg_bvss_levels(cpg_bvss* b, const cpg_bvss_opts* opts, const int32_t
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   float ms = 0.f;
   if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   BCK(e, "BVSS levels");
   if (c.err == kDevTimeout) return bfail(b, CPG_ERR_TIMEOUT, "BVSS levels: grid barrier wait ran out");
   if (stats) {
@@ -364,9 +372,7 @@ cpg_status cpg_bvss_discover_pairs(cpg_bvss* b, const cpg_bvss_opts* opts,
   BCK(grow(b->d_io, static_cast<size_t>(n_sources) * 4), "alloc BVSS sources");
   BCK(grow(b->d_out, static_cast<size_t>(std::max<int64_t>(max_pairs, 1)) * 8), "alloc BVSS pairs");
   cudaStream_t s = static_cast<cudaStream_t>(o.stream);
-  cudaEvent_t e0, e1;
-  BCK(cudaEventCreate(&e0), "event");
-  BCK(cudaEventCreate(&e1), "event");
+  const cudaEvent_t e0 = b->ev[0], e1 = b->ev[1];
   cudaError_t e = cudaSuccess;
   if (n_sources) e = cudaMemcpyAsync(b->d_io.p, sources, static_cast<size_t>(n_sources) * 4,
                                      cudaMemcpyHostToDevice, s);
@@ -377,7 +383,7 @@ cpg_status cpg_bvss_discover_pairs(cpg_bvss* b, const cpg_bvss_opts* opts,
         static_cast<int32_t*>(b->d_out.p), max_pairs, static_cast<unsigned int*>(b->d_scratch.p),
         static_cast<BvssCounters*>(b->d_ctr.p), dispatch(o), s));
   if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-  BvssCounters c{};
+  BvssCounters& c = *b->counters;
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&c, b->d_ctr.p, sizeof(c), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -387,8 +393,6 @@ cpg_status cpg_bvss_discover_pairs(cpg_bvss* b, const cpg_bvss_opts* opts,
     e = cudaMemcpy(pairs, b->d_out.p, static_cast<size_t>(got) * 8, cudaMemcpyDeviceToHost);
   float ms = 0.f;
   if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   BCK(e, "BVSS pairs");
   *n_pairs = total;
   if (stats) {
