@@ -1,5 +1,7 @@
 // Persistent query engine for sm_100a: whole critical-path queries on the
-// device, for one query or a batch of them, in one cooperative launch.
+// device, for one query or a batch of them.  Every query starts on a block of
+// its own (engine_block_kernel), where small ones end; one cooperative launch
+// (engine_kernel) goes on with the others.
 //
 // Per query it reproduces the reference's report_paths after the suffix tree
 // (gpucpg/gpucpg.cu:18502-21366) for SHORT_LONG:
@@ -10,10 +12,12 @@
 //               stopping rule of the SHORT_LONG driver (19134-20850)
 //   output      the K cheapest non-zero paths, ascending (21323-21360)
 // The split raises, the closures between them, the top-K select and the
-// segmented sort run back to back between bounded grid barriers; the host
-// launches once and reads the results.
+// segmented sort run back to back between block barriers, or bounded grid
+// barriers; the host launches both and reads the results.  A query that
+// outgrows its block is the exception: the host then seeds it again
+// (seed_left_kernel) and launches the grid for it.
 //
-// Work layout: pending path-graph items of all queries share one pile (the
+// Work layout of the grid launch: pending path-graph items of all queries share one pile (the
 // query id rides in the top bits of Item::j), accepted paths share one store
 // (pq[] holds their query); per-query state lives in EngineQuery.  Selection
 // is a three-pass radix select per query over kSelBins-bin histograms;

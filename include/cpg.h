@@ -104,8 +104,12 @@ typedef struct {
                                build on large graphs, else by the building
                                warp right after each build), 1 = always by the
                                building warp, 2 = always in the heap phase */
-  int32_t engine_ctas;      /* single queries: CTAs of the engine launch
-                               (0 = chosen from k) */
+  int32_t engine_ctas;      /* CTAs of a single query's grid launch (0 =
+                               chosen from k).  Every query starts on a block
+                               of its own, and small ones end there; a value
+                               above 0 sends every query, in the batched and
+                               served forms too, on to the grid launch (A/B
+                               checks) */
   int32_t sfxt_claim_sets;  /* dataflow build: how warps take work-queue
                                slots.  0 = default (claimed, 8 sets), -1 =
                                static (warp w takes slots w, w + W, ...; A/B
@@ -415,8 +419,8 @@ cpg_status cpg_select_topk(const float* d_costs, int64_t n, int64_t k,
  *  - The scratch (about 2.2 MiB) is reserved on every GPU that loads the
  *    library and kept until the process exits.
  *  - No call can run inside a stream capture: every call reads the count of
- *    non-zero costs back to the host partway through and synchronises
- *    `stream` before it returns.
+ *    non-zero costs back to the host at its end and synchronises `stream` for
+ *    it before it returns.
  *  - The first call on a device looks up the scratch's device address (with
  *    that device current).  The address is kept for the life of the
  *    process: after cudaDeviceReset on that device the module is loaded
