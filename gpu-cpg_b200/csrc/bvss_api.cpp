@@ -38,10 +38,7 @@ struct cpg_bvss {
   std::string err;
   int device = -1;  // device holding the copy below
   Buf d_ptr, d_v2r, d_cnt, d_rows, d_masks, d_scratch, d_ctr, d_io, d_out;
-  // around the device work of a run, and where its counters come back (a call
-  // of few sources is bound by what it does besides the kernels)
-  cudaEvent_t ev[2] = {};
-  BvssCounters* counters = nullptr;  // pinned
+  cudaEvent_t ev[2] = {};  // around the device work of a run
 };
 
 namespace {
@@ -72,8 +69,6 @@ void drop_device(cpg_bvss* b) {
     if (x) cudaEventDestroy(x);
     x = nullptr;
   }
-  if (b->counters) cudaFreeHost(b->counters);
-  b->counters = nullptr;
   b->device = -1;
 }
 
@@ -88,7 +83,6 @@ Status upload(cpg_bvss* b, int device) {
   if (b->device == device) return CPG_OK;
   drop_device(b);
   for (cudaEvent_t& x : b->ev) BCK(cudaEventCreate(&x), "event");
-  BCK(cudaMallocHost(&b->counters, sizeof(BvssCounters)), "alloc BVSS");
   const HostBvss& h = b->hb;
   BCK(grow(b->d_ptr, h.ptr.size() * 4), "alloc BVSS");
   BCK(grow(b->d_v2r, h.v2r.size() * 4), "alloc BVSS");
@@ -332,7 +326,7 @@ cpg_status cpg_bvss_levels(cpg_bvss* b, const cpg_bvss_opts* opts, const int32_t
         static_cast<BvssCounters*>(b->d_ctr.p), dispatch(o),
         o.spin_limit ? o.spin_limit : kBvssSpinLimit, o.device, s));
   if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-  BvssCounters& c = *b->counters;
+  BvssCounters c{};
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&c, b->d_ctr.p, sizeof(c), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && h.n_rows)
@@ -383,7 +377,7 @@ cpg_status cpg_bvss_discover_pairs(cpg_bvss* b, const cpg_bvss_opts* opts,
         static_cast<int32_t*>(b->d_out.p), max_pairs, static_cast<unsigned int*>(b->d_scratch.p),
         static_cast<BvssCounters*>(b->d_ctr.p), dispatch(o), s));
   if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-  BvssCounters& c = *b->counters;
+  BvssCounters c{};
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(&c, b->d_ctr.p, sizeof(c), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
