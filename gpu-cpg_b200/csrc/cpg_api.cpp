@@ -1107,8 +1107,8 @@ int try_query(cpg_handle* h, unsigned long long k) {
 }
 
 // ---- query engine: prepare (allocate, upload the query table), enqueue
-// (asynchronous and capturable: memsets and one cooperative launch) and
-// finish (read counters back, map errors).
+// (asynchronous and capturable: memsets, the launch of the blocks and the grid
+// launch) and finish (read counters back, map errors).
 
 // Which queries their blocks answer whole, where each query's costs go, and
 // every block's share of the path store and piles, the queries that go on to

@@ -383,8 +383,10 @@ int launch_promote(const Item* pend_in, unsigned long long n_in, float lim,
 // ---------------------------------------------------------------- engine
 // The persistent query engine (engine.cu) runs whole queries on the device:
 // root seeding, every split raise, the closures, the final top-K select and
-// the segmented sort, for any number of queries over one device graph, in
-// one cooperative launch with no host round trip.
+// the segmented sort, for any number of queries over one device graph: a
+// launch with a block per query, then a cooperative launch for those that do
+// not end there, with no host round trip (but for a query that outgrew its
+// block).
 constexpr int kMaxQueries = 4096;   // Item.j carries the query id in 12 bits
 constexpr int kJBits = 20;          // ... and the deviation index in 20 bits
 constexpr unsigned kJMask = (1u << kJBits) - 1u;
